@@ -137,6 +137,11 @@ def gemm_bf16(x, w, out=None, out_dtype=torch.bfloat16, accumulate=False, bn=0, 
         out = torch.empty(*x.shape[:-1], n, dtype=out_dtype, device=x.device)
     o2 = out.reshape(-1, n) if out.is_contiguous() else out
     assert o2.stride(-1) == 1
+    if bn == 0 and splits == 0 and act not in GATES and _many_rows(x2, w, m, n, k, 1):
+        nv.call("gemm_prefill", nv.ptr(x2), nv.ptr(w), nv.ptr(o2), I(m), I(n), I(k), I(x2.stride(0)), I(w.stride(0)),
+                I(o2.stride(0)), I(1 if out.dtype == torch.float32 else 0), I(1 if accumulate else 0), I(ACTS[act]), F(0.0), I(1),
+                I(NUM_SMS_HINT))
+        return out
     bn, splits = pick_tiling(m, n, (k + 63) // 64, 1, False, bn, splits)
     ws, cnt = _ws(m, n, bn, 1, splits, x.device)
     nv.call("gemm_bf16", nv.ptr(x2), nv.ptr(w), nv.ptr(o2), I(m), I(n), I(k), I(x2.stride(0)), I(w.stride(0)),
@@ -151,11 +156,19 @@ def _tma_ok(x2, w, k: int) -> bool:
             and x2.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
-PREFILL_MIN_TILES = 100     # 128 x 256 output tiles from which the persistent kernel (csrc/gemm_prefill.cu) fills the GPU
+# 128 x 256 output tiles from which the persistent kernel (csrc/gemm_prefill.cu) fills the GPU: 8 192 rows of the grouped
+# 8 x (4 096 -> 1 024) projection take 379 us there and 676 us on one CTA per 128 x 128 tile (gemm_tcgen05.cu), whose epilogue
+# nothing overlaps; 4 096 -> 2 560 with 32-bit results 143 and 245 us
+PREFILL_MIN_TILES = 100
 
 
 def prefill_tiles(m: int, n: int, groups: int) -> int:
     return -(-m // 128) * -(-n // 256) * groups if m > 128 else 0
+
+
+def _many_rows(x2, w, m: int, n: int, k: int, groups: int) -> bool:
+    """Whether the persistent kernel takes this bf16 projection."""
+    return prefill_tiles(m, n, groups) >= PREFILL_MIN_TILES and _tma_ok(x2, w, k)
 
 
 def linear(x, w, out=None, out_dtype=None, accumulate=False, act=None, limit=0.0):
@@ -181,7 +194,7 @@ def grouped_linear(x, w, groups: int, out=None, out_dtype=None, accumulate=False
     assert w.dtype == torch.bfloat16 and w.stride(-1) == 1 and x.stride(-1) == 1 and out.stride(-1) == 1
     f32 = I(1 if out.dtype == torch.float32 else 0)
     if _tma_ok(x, w, k):
-        if prefill_tiles(t, n, groups) >= PREFILL_MIN_TILES:
+        if _many_rows(x, w, t, n, k, groups):
             nv.call("gemm_prefill", nv.ptr(x), nv.ptr(w), nv.ptr(out), I(t), I(n), I(k), I(x.stride(0)), I(w.stride(0)),
                     I(out.stride(0)), f32, I(1 if accumulate else 0), I(ACTS[act]), F(limit), I(groups), I(NUM_SMS_HINT))
             return out
@@ -253,6 +266,10 @@ def gemm_bf16_grouped(x, w, groups: int, out=None):
     assert x.is_contiguous() and w.is_contiguous() and x.dtype == torch.bfloat16
     if out is None:
         out = torch.empty(t, groups * n, dtype=x.dtype, device=x.device)
+    if out.dtype == torch.bfloat16 and _many_rows(x, w, t, n, k, groups):
+        nv.call("gemm_prefill", nv.ptr(x), nv.ptr(w), nv.ptr(out), I(t), I(n), I(k), I(x.stride(0)), I(w.stride(0)),
+                I(out.stride(0)), I(0), I(0), I(0), F(0.0), I(groups), I(NUM_SMS_HINT))
+        return out
     bn, splits = pick_tiling(t, n, (k + 63) // 64, groups, False, 0, 0)
     ws, cnt = _ws(t, n, bn, groups, splits, x.device)
     nv.call("gemm_bf16", nv.ptr(x), nv.ptr(w), nv.ptr(out), I(t), I(n), I(k), I(x.stride(0)), I(w.stride(0)),

@@ -99,3 +99,28 @@ def test_gemm_bf16_grouped(t, groups):
     y = gemm.gemm_bf16_grouped(x, w, groups)
     ref = gemm.gemm_bf16_grouped(x.cpu(), w.cpu(), groups)
     assert torch.allclose(y.float().cpu(), ref.float(), rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("m,n,k,groups", [(8192, 264, 64, 1), (3333, 1000, 136, 1), (12801, 256, 200, 1), (1700, 1024, 192, 8),
+                                          (1665, 296, 72, 4)])
+def test_many_rows_on_the_persistent_kernel(m, n, k, groups):
+    """The persistent kernel gives what one CTA per tile gives: row and column remainders, K that ends inside a tile, strided
+    rows, 32-bit results, addition to a result.  Both add a tile's products in the same order, so the results are equal."""
+    assert gemm.prefill_tiles(m, n, groups) >= gemm.PREFILL_MIN_TILES
+    g = torch.Generator(device="cuda").manual_seed(m)
+    wide = torch.randn(m, k * groups + 8, generator=g, device="cuda").bfloat16()
+    w = torch.randn(n * groups, k, generator=g, device="cuda").bfloat16()
+    x = wide[:, :k * groups]
+    want = torch.einsum("tgk,gnk->tgn", x.reshape(m, groups, k).float(), w.view(groups, n, k).float()).reshape(m, -1)
+    if groups > 1:
+        got = gemm.gemm_bf16_grouped(x.contiguous(), w, groups)
+        assert ((got.float() - want).norm() / want.norm()).item() < 3e-3        # one rounding to bf16: at most 2^-9 each
+        return
+    for dtype in (torch.bfloat16, torch.float32):
+        assert torch.equal(gemm.gemm_bf16(x, w, out_dtype=dtype), gemm.gemm_bf16(x, w, out_dtype=dtype, bn=128, splits=1))
+        a = torch.randn(m, n + 8, generator=g, device="cuda").to(dtype)
+        b = a.clone()
+        gemm.gemm_bf16(x, w, out=a[:, :n], accumulate=True, act="relu2")
+        gemm.gemm_bf16(x, w, out=b[:, :n], accumulate=True, act="relu2", bn=128, splits=1)
+        assert torch.equal(a, b)
+    assert ((gemm.gemm_bf16(x, w, out_dtype=torch.float32) - want).norm() / want.norm()).item() < 1e-4
