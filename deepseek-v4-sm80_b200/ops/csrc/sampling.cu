@@ -45,64 +45,18 @@ __device__ __forceinline__ unsigned long long block_scan_u64(unsigned long long 
   return x - v + (w ? wt[w - 1] : 0ull);
 }
 
-__global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ logits, int v,
-                                                      const float* __restrict__ temperature,
-                                                      const int* __restrict__ top_k, const float* __restrict__ top_p,
-                                                      const float* __restrict__ uniform,
-                                                      const int* __restrict__ mask_ids, int n_mask,
-                                                      long long* __restrict__ out) {
-  pdl_entry();
-  __shared__ float sf[32];
+// Any row: the key of the last kept rank byte by byte, each byte a pass over the whole row.  Rows that the histogram below cannot
+// order come here: a maximum or a temperature that is not finite, values that are not numbers, more entries in the last kept bin
+// than its list holds (equal logits above all).
+template <class V>
+__device__ __noinline__ int sample_exhaustive(V val, int v, float mx, int amax, float temp, int tk, float tp, float u) {
   __shared__ int si[32];
   __shared__ unsigned long long wt[32];
   __shared__ unsigned long long hmass[256];
   __shared__ int hcnt[256];
   __shared__ int sh_bin, sh_cnt_above;
   __shared__ unsigned long long sh_mass_above;
-  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const float* row = logits + (size_t)b * v;
-  const int* mrow = mask_ids ? mask_ids + (size_t)b * n_mask : nullptr;
-  auto val = [&](int i) -> float {
-    float x = row[i];
-    for (int m = 0; m < n_mask; ++m)
-      if (mrow[m] == i) x = -INFINITY;
-    return x;
-  };
-  // argmax (lowest id wins ties) -- also the softmax max
-  float best = -INFINITY;
-  int bi = 0x7fffffff;
-  for (int i = tid; i < v; i += 1024) {
-    const float x = val(i);
-    if (x > best || (x == best && i < bi)) best = x, bi = i;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (ob > best || (ob == best && oi < bi)) best = ob, bi = oi;
-  }
-  if (lane == 0) sf[w] = best, si[w] = bi;
-  __syncthreads();
-  if (w == 0) {
-    best = sf[lane], bi = si[lane];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) best = ob, bi = oi;
-    }
-    if (lane == 0) sf[0] = best, si[0] = bi;
-  }
-  __syncthreads();
-  const float mx = sf[0];
-  const int amax = si[0];
-  const float temp = temperature ? temperature[b] : 0.f;
-  const int tk = top_k ? top_k[b] : -1;
-  const float tp = top_p ? top_p[b] : 1.f;
-  if (temp <= 0.f || tk == 1) {
-    if (tid == 0) out[b] = amax;
-    return;
-  }
+  const int tid = threadIdx.x, lane = tid & 31;
   const float inv_t = 1.f / temp;
   // Z in fixed point of exp((x - mx)/T)  (each term <= 1)
   unsigned long long zl = 0;
@@ -181,7 +135,6 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
   // kept: key > prefix, plus threshold ties in id order while count < k and mass before < p.
   // Every thread owns a contiguous range of ids, so "in id order" needs three block scans in total (ties before the
   // thread, tie mass before it, kept mass before it) and sequential walks inside the thread's own range.
-  const float u = uniform ? uniform[b] : 0.5f;
   const int per = (v + 1023) / 1024;
   const int i_lo = min(tid * per, v), i_hi = min(i_lo + per, v);
   unsigned long long my_eq_mass = 0;
@@ -223,7 +176,290 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
     if (id != ~0ull) si[1] = (int)id;
   }
   __syncthreads();
-  if (tid == 0) out[b] = si[1];
+  return si[1];
+}
+
+// Sums and a list per row of the route below.
+constexpr int kBins = 2048;      // of (mx - x) / T, 1/64 wide: from 28 on (the last 256 bins) a mass is 0 in 2^-40
+constexpr int kList = 4096;      // entries of the last kept bin that can be put in order
+constexpr int kTopList = 256;    // top_k up to which the threads' maxima bound the kept set
+
+struct SampleSmem {
+  union {
+    struct {
+      uint32_t lo[kBins], hi[kBins];   // mass of a bin
+      int cnt[kBins];
+    } h;
+    unsigned long long list[kList];
+  };
+  unsigned long long wt[32], seg[32];
+  unsigned long long mass_above, last;
+  int n, bin, cnt_above, found;
+};
+
+// list[0..n) in descending order, n <= kList; all 1024 threads.
+__device__ __forceinline__ void sort_list(unsigned long long* list, int n) {
+  int p = 32;
+  while (p < n) p <<= 1;
+  __syncthreads();
+  for (int i = n + threadIdx.x; i < p; i += 1024) list[i] = 0ull;
+  __syncthreads();
+  for (int size = 2; size <= p; size <<= 1)
+    for (int step = size >> 1; step > 0; step >>= 1) {
+      for (int i = threadIdx.x; i < (p >> 1); i += 1024) {
+        const int a = 2 * i - (i & (step - 1)), b = a + step;
+        const unsigned long long x = list[a], y = list[b];
+        if ((x < y) == ((a & size) == 0)) list[a] = y, list[b] = x;
+      }
+      __syncthreads();
+    }
+}
+
+__device__ __forceinline__ float key_value(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
+
+// What bounds it: passes over the row, which the L2 holds after the first (128 rows of 129 280 floats: 66 MB).  A warp reads one
+// 32nd of the row, 16 bytes a lane and four loads in flight.  Two to three passes do: the maximum; the sum of the masses together
+// with a histogram of (mx - x) / T, or, for a top_k of at most 256, with the list of what reaches the k-th largest of the threads'
+// own maxima (at least k entries do); then, behind a histogram, the masses that the last kept bin's order decides.
+// Only that bin's entries, about 200 of them for logits of a spread of 2.5, or that list are put in order.  The pass that finds the
+// sample reads the one 32nd that it falls into.  128 rows of 129 280 at top_k 50 and top_p 0.95 take 55 us; the four passes of the
+// descent, three walks over 126 consecutive ids a thread and the passes before them took 620 us.
+__global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ logits, int v,
+                                                      const float* __restrict__ temperature,
+                                                      const int* __restrict__ top_k, const float* __restrict__ top_p,
+                                                      const float* __restrict__ uniform,
+                                                      const int* __restrict__ mask_ids, int n_mask,
+                                                      long long* __restrict__ out) {
+  pdl_entry();
+  using u64 = unsigned long long;
+  __shared__ float sf[32];
+  __shared__ int si[32], sbad;
+  __shared__ SampleSmem sm;
+  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const float* row = logits + (size_t)b * v;
+  const int* mrow = mask_ids ? mask_ids + (size_t)b * n_mask : nullptr;
+  auto masked = [&](float x, int i) -> float {
+    for (int m = 0; m < n_mask; ++m)
+      if (mrow[m] == i) x = -INFINITY;
+    return x;
+  };
+  // f(x, id) over this warp's ids [lo, hi); whole groups of four that start on 16 bytes are one load
+  const int per_warp = ((v + 127) / 128) * 4;
+  const int lo = min(w * per_warp, v), hi = min(lo + per_warp, v);
+  auto each = [&](auto f) {
+    const int head = min(hi, lo + (int)((4 - (((uintptr_t)(row + lo) >> 2) & 3)) & 3));
+    if (lo + lane < head) f(masked(row[lo + lane], lo + lane), lo + lane);
+    const float4* r4 = reinterpret_cast<const float4*>(row + head);
+    const int n4 = (hi - head) >> 2;
+    int i = lane;
+    for (; i + 96 < n4; i += 128) {
+      float4 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] = r4[i + 32 * u];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int id = head + 4 * (i + 32 * u);
+        f(masked(x[u].x, id), id), f(masked(x[u].y, id + 1), id + 1);
+        f(masked(x[u].z, id + 2), id + 2), f(masked(x[u].w, id + 3), id + 3);
+      }
+    }
+    for (; i < n4; i += 32) {
+      const float4 x = r4[i];
+      const int id = head + 4 * i;
+      f(masked(x.x, id), id), f(masked(x.y, id + 1), id + 1), f(masked(x.z, id + 2), id + 2), f(masked(x.w, id + 3), id + 3);
+    }
+    const int tail = head + 4 * n4 + lane;
+    if (tail < hi) f(masked(row[tail], tail), tail);
+  };
+  // argmax (lowest id wins ties) -- also the softmax max
+  if (tid == 0) sbad = 0, sm.n = 0;
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+  bool nan = false;
+  each([&](float x, int i) {
+    nan |= x != x;
+    if (x > best || (x == best && i < bi)) best = x, bi = i;
+  });
+  const float own = best;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    if (ob > best || (ob == best && oi < bi)) best = ob, bi = oi;
+  }
+  if (lane == 0) sf[w] = best, si[w] = bi;
+  __syncthreads();
+  if (nan) sbad = 1;
+  if (w == 0) {
+    best = sf[lane], bi = si[lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (ob > best || (ob == best && oi < bi)) best = ob, bi = oi;
+    }
+    if (lane == 0) sf[0] = best, si[0] = bi;
+  }
+  __syncthreads();
+  const float mx = sf[0];
+  const int amax = si[0];
+  const float temp = temperature ? temperature[b] : 0.f;
+  const int tk = top_k ? top_k[b] : -1;
+  const float tp = top_p ? top_p[b] : 1.f;
+  if (temp <= 0.f || tk == 1) {
+    if (tid == 0) out[b] = amax;
+    return;
+  }
+  const float u = uniform ? uniform[b] : 0.5f;
+  const float inv_t = 1.f / temp;
+  auto exhaustive = [&]() {
+    const int id = sample_exhaustive([&](int i) { return masked(row[i], i); }, v, mx, amax, temp, tk, tp, u);
+    if (tid == 0) out[b] = id;
+  };
+  if (sbad || !isfinite(mx) || !isfinite(inv_t)) {
+    exhaustive();
+    return;
+  }
+  auto mass = [&](float x) { return fx(expf((x - mx) * inv_t)); };
+  auto entry = [](uint32_t key, int id) { return (u64)key << 32 | (0xffffffffu - (uint32_t)id); };   // larger: earlier in the order
+  const int k_limit = tk > 0 ? tk : 0x7fffffff;
+  const bool keep_all = tk <= 0 && tp >= 1.f, few = tk > 0 && tk <= kTopList;
+  u64 zl = 0, ztot;
+  u64 last = 0;              // the last kept entry: kept are those not below it
+  bool none = false;         // top_p leaves nothing
+  if (few) {
+    // at least k of the threads' maxima, so at least k values, are not below their k-th
+    sm.list[tid] = (u64)okey(own) << 32 | (uint32_t)tid;
+    sort_list(sm.list, 1024);
+    const uint32_t bound = (uint32_t)(sm.list[tk - 1] >> 32);
+    __syncthreads();
+    each([&](float x, int i) {
+      zl += mass(x);
+      const uint32_t key = okey(x);
+      if (key >= bound) {
+        const int at = atomicAdd(&sm.n, 1);
+        if (at < kList) sm.list[at] = entry(key, i);
+      }
+    });
+  } else if (keep_all) {
+    each([&](float x, int) { zl += mass(x); });
+  } else {
+    for (int i = tid; i < kBins; i += 1024) sm.h.lo[i] = sm.h.hi[i] = 0, sm.h.cnt[i] = 0;
+    __syncthreads();
+    const bool counted = tk > 0;
+    each([&](float x, int) {
+      const u64 m = mass(x);
+      zl += m;
+      const int bin = min(__float2int_rz(fminf((mx - x) * inv_t, 1e6f) * 64.f), kBins - 1);
+      const uint32_t m_lo = (uint32_t)m;
+      uint32_t m_hi = (uint32_t)(m >> 32);
+      if (m_lo && atomicAdd(&sm.h.lo[bin], m_lo) + m_lo < m_lo) ++m_hi;    // a carry
+      if (m_hi) atomicAdd(&sm.h.hi[bin], m_hi);
+      if (counted) atomicAdd(&sm.h.cnt[bin], 1);
+    });
+  }
+  block_scan_u64(zl, sm.wt, ztot);
+  const u64 p_limit = tp >= 1.f ? ~0ull : (u64)((double)ztot * (double)tp);
+  u64 mass_above = 0;
+  int cnt_above = 0, bin_last = -1;
+  if (!few && !keep_all) {
+    // the first bin, from the largest values on, with which the count reaches k or the mass p
+    const int b0 = 2 * tid;
+    const u64 m0 = (u64)sm.h.hi[b0] << 32 | sm.h.lo[b0], m1 = (u64)sm.h.hi[b0 + 1] << 32 | sm.h.lo[b0 + 1];
+    const int c0 = sm.h.cnt[b0], c1 = sm.h.cnt[b0 + 1];
+    if (tid == 0) sm.bin = -1;
+    u64 tot;
+    const u64 m_before = block_scan_u64(m0 + m1, sm.wt, tot);
+    const int c_before = (int)block_scan_u64((u64)(c0 + c1), sm.wt, tot);
+    auto ends = [&](int c, u64 m) { return c >= k_limit || m >= p_limit; };
+    const bool before = tid > 0 && ends(c_before, m_before);
+    if (!before && ends(c_before + c0, m_before + m0))
+      sm.bin = b0, sm.mass_above = m_before, sm.cnt_above = c_before;
+    else if (!before && ends(c_before + c0 + c1, m_before + m0 + m1))
+      sm.bin = b0 + 1, sm.mass_above = m_before + m0, sm.cnt_above = c_before + c0;
+    __syncthreads();
+    bin_last = sm.bin;
+    if (bin_last >= 0) mass_above = sm.mass_above, cnt_above = sm.cnt_above;
+    __syncthreads();
+  }
+  // the kept mass of each warp's ids; entries of the last bin are listed and counted once their order is known
+  u64 own_mass = 0;
+  if (keep_all || (!few && bin_last < 0)) {
+    own_mass = zl;
+  } else if (!few) {
+    each([&](float x, int i) {
+      const int bin = min(__float2int_rz(fminf((mx - x) * inv_t, 1e6f) * 64.f), kBins - 1);
+      if (bin < bin_last) own_mass += mass(x);
+      if (bin == bin_last) {
+        const int at = atomicAdd(&sm.n, 1);
+        if (at < kList) sm.list[at] = entry(okey(x), i);
+      }
+    });
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) own_mass += __shfl_xor_sync(0xffffffffu, own_mass, o);
+  if (lane == 0) sm.seg[w] = own_mass;
+  __syncthreads();
+  const int n = sm.n;
+  if (n > kList) {
+    exhaustive();
+    return;
+  }
+  if (n > 0) {
+    sort_list(sm.list, n);
+    u64 e[4], m[4], before, tot;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      e[j] = 4 * tid + j < n ? sm.list[4 * tid + j] : 0ull;
+      m[j] = 4 * tid + j < n ? mass(key_value((uint32_t)(e[j] >> 32))) : 0ull;
+    }
+    if (tid == 0) sm.last = 0ull;
+    before = mass_above + block_scan_u64(m[0] + m[1] + m[2] + m[3], sm.wt, tot);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int r = 4 * tid + j;
+      auto kept = [&](int rank, u64 mass_before) { return rank < n && cnt_above + rank < k_limit && mass_before < p_limit; };
+      if (kept(r, before)) {
+        atomicAdd(&sm.seg[(0xffffffffu - (uint32_t)e[j]) / per_warp], m[j]);
+        if (!kept(r + 1, before + m[j])) sm.last = e[j];
+      }
+      before += m[j];
+    }
+    __syncthreads();
+    last = sm.last;
+    none = last == 0ull;
+  }
+  // the warp's ids that the running kept mass passes the target in, and then the id
+  u64 kept_total;
+  const u64 kept_before = block_scan_u64(lane == 0 ? sm.seg[w] : 0ull, sm.wt, kept_total);
+  u64 target = (u64)((double)u * (double)kept_total);
+  if (target >= kept_total && kept_total > 0) target = kept_total - 1;
+  if (tid == 0) sm.found = amax, sm.bin = -1;
+  __syncthreads();
+  if (lane == 0 && !none && target >= kept_before && target < kept_before + sm.seg[w]) sm.bin = w, sm.mass_above = kept_before;
+  __syncthreads();
+  if (sm.bin >= 0) {
+    const int first = sm.bin * per_warp, end = min(first + per_warp, v), per = (per_warp + 1023) / 1024;
+    const int a = min(first + tid * per, end), z = min(a + per, end);
+    auto kept_mass = [&](int i) -> u64 {
+      const float x = masked(row[i], i);
+      return entry(okey(x), i) >= last ? mass(x) : 0ull;
+    };
+    u64 mine = 0, tot;
+    for (int i = a; i < z; ++i) mine += kept_mass(i);
+    u64 run = sm.mass_above + block_scan_u64(mine, sm.wt, tot);
+    if (target >= run && target < run + mine)
+      for (int i = a; i < z; ++i) {
+        const u64 pm = kept_mass(i);
+        if (run <= target && run + pm > target) {
+          sm.found = i;
+          break;
+        }
+        run += pm;
+      }
+    __syncthreads();
+  }
+  if (tid == 0) out[b] = sm.found;
 }
 
 }  // namespace
