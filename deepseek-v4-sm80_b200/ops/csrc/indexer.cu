@@ -7,8 +7,8 @@
 //
 // top-k keeps the reference's contract (csrc/jit/dsv4_topk_v1.cu:275-479): rows shorter than k keep every entry,
 // a non-finite score invalidates the row (len = -1), ties at the threshold are resolved towards the lower index.
-// The selection is a 4-pass 8-bit radix select on order-preserving keys followed by an ordered compaction, so
-// the result is deterministic and comes out sorted by index (attention does not depend on the order).
+// The selection finds the last selected entry in the order (score descending, index ascending) and writes what is not below it,
+// so the result is deterministic and comes out sorted by index (attention does not depend on the order).
 #include "common.cuh"
 
 namespace {
@@ -83,8 +83,9 @@ __device__ __forceinline__ uint32_t order_key(float f) {
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
+// Exclusive prefix of v over the NT threads of the CTA, total = their sum.
+template <int NT>
 __device__ __forceinline__ int block_excl_scan(int v, int* warp_tot, int& total) {
-  // 1024 threads; returns exclusive prefix of v, total = block sum
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int x = v;
 #pragma unroll
@@ -96,85 +97,212 @@ __device__ __forceinline__ int block_excl_scan(int v, int* warp_tot, int& total)
   if (lane == 31) warp_tot[w] = x;
   __syncthreads();
   if (w == 0) {
-    int s = warp_tot[lane];
+    int s = lane < NT / 32 ? warp_tot[lane] : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, s, o);
       if (lane >= o) s += y;
     }
-    warp_tot[lane] = s;
+    if (lane < NT / 32) warp_tot[lane] = s;
   }
   __syncthreads();
-  total = warp_tot[31];
+  total = warp_tot[NT / 32 - 1];
   return x - v + (w ? warp_tot[w - 1] : 0);
 }
 
-__global__ void __launch_bounds__(1024) topk_kernel(const float* __restrict__ logits, int width,
-                                                    const int* __restrict__ pos, int* __restrict__ idx,
-                                                    int* __restrict__ out_len, int k) {
+constexpr int kTopBins = 2048;   // equal parts of the row's range of values
+constexpr int kTopList = 512;    // entries of the k-th one's part that are put in order
+
+// One CTA per row.  The k-th largest value lies in one of 2 048 equal parts of the row's range of values, found by counting; the few
+// entries of that part (about ten of 8 000 normal scores) are ranked against each other, which gives the last selected entry, and
+// one ordered pass writes what is not below it.  A row whose part holds more than kTopList entries (equal scores, one far outlier)
+// finds the k-th key byte by byte instead.  The four passes read registers: V float4 a thread hold the row of up to NT * 4 * V
+// entries, a warp consecutive ones (V = 0: longer rows, read again by each pass).
+// Bound by the steps of one row, not by its bytes: rows in flight hide them (512 threads for the rows of prompts: three CTAs an SM).
+// 4 096 rows of about 7 700: 130 us, against 775 us with four passes over key bytes whose 256 counts one thread walked.
+template <int NT, int V>
+__global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_kernel(const float* __restrict__ logits, int width,
+                                                  const int* __restrict__ pos, int* __restrict__ idx,
+                                                  int* __restrict__ out_len, int k) {
   pdl_entry();
-  __shared__ int hist[256];
+  __shared__ int hist[kTopBins];
+  __shared__ unsigned long long list[kTopList];
   __shared__ int wt[32];
-  __shared__ int sh_bad, sh_bin, sh_rem;
-  const int t = blockIdx.x, tid = threadIdx.x;
+  __shared__ float smin[32], smax[32];
+  __shared__ int sh_bad, sh_bin, sh_above, sh_n;
+  __shared__ unsigned long long sh_last;
+  const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int n = min((pos[t] + 1) >> 2, width);
   int* oi = idx + (size_t)t * k;
   if (n <= k) {
-    for (int i = tid; i < k; i += 1024) oi[i] = i < n ? i : -1;
+    for (int i = tid; i < k; i += NT) oi[i] = i < n ? i : -1;
     if (tid == 0) out_len[t] = n;
     return;
   }
   const float* row = logits + (size_t)t * width;
-  if (tid == 0) sh_bad = 0;
+  const bool vec = ((reinterpret_cast<uintptr_t>(logits) & 15) | (width & 3)) == 0;
+  auto load = [&](int i) -> float4 {   // entries i .. i + 3 (i a multiple of four); those from n on are not looked at
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (vec) {
+      if (i < n) x = *reinterpret_cast<const float4*>(row + i);
+    } else {
+      if (i < n) x.x = row[i];
+      if (i + 1 < n) x.y = row[i + 1];
+      if (i + 2 < n) x.z = row[i + 2];
+      if (i + 3 < n) x.w = row[i + 3];
+    }
+    return x;
+  };
+  // a warp's entries: `per` consecutive ones, 128 at a time
+  const int per = V ? 128 * V : (((n + NT / 32 - 1) / (NT / 32) + 127) & ~127);
+  const int first = w * per + 4 * lane;
+  float4 held[V ? V : 1];
+  if (V) {
+#pragma unroll
+    for (int u = 0; u < V; ++u) held[u] = load(first + 128 * u);
+  }
+  auto each4 = [&](auto f) {           // f(four values, id of the first); a warp's lanes stay together
+    if (V) {
+#pragma unroll
+      for (int u = 0; u < V; ++u) f(held[u], first + 128 * u);
+    } else {
+      for (int i = 0; i < per && w * per + i < n; i += 128) f(load(first + i), first + i);
+    }
+  };
+  auto each = [&](auto f) {
+    each4([&](const float4& x, int i) {
+      if (i < n) f(x.x, i);
+      if (i + 1 < n) f(x.y, i + 1);
+      if (i + 2 < n) f(x.z, i + 2);
+      if (i + 3 < n) f(x.w, i + 3);
+    });
+  };
+  for (int i = tid; i < kTopBins; i += NT) hist[i] = 0;
+  if (tid == 0) sh_bad = 0, sh_n = 0;
+  float mn = INFINITY, mx = -INFINITY;
+  bool bad = false;
+  each([&](float x, int) { bad |= !isfinite(x), mn = fminf(mn, x), mx = fmaxf(mx, x); });
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o)), mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane == 0) smin[w] = mn, smax[w] = mx;
   __syncthreads();
-  int bad = 0;
-  for (int i = tid; i < n; i += 1024) bad |= !isfinite(row[i]);
   if (bad) sh_bad = 1;
+  for (int i = 0; i < NT / 32; ++i) mn = fminf(mn, smin[i]), mx = fmaxf(mx, smax[i]);
   __syncthreads();
   if (sh_bad) {
-    for (int i = tid; i < k; i += 1024) oi[i] = -1;
+    for (int i = tid; i < k; i += NT) oi[i] = -1;
     if (tid == 0) out_len[t] = -1;
     return;
   }
-  uint32_t prefix = 0, mask = 0;
-  int rem = k;  // how many still to take among elements matching the prefix
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    for (int i = tid; i < 256; i += 1024) hist[i] = 0;
-    __syncthreads();
-    for (int i = tid; i < n; i += 1024) {
-      const uint32_t key = order_key(row[i]);
-      if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 0xff], 1);
+  // part 0 holds the largest values; a range that overflows or has no width puts all into one part, which the list then refuses
+  const float scale = (float)kTopBins / (mx - mn);
+  auto part = [&](float x) { return min(max(__float2int_rz((mx - x) * scale), 0), kTopBins - 1); };
+  auto entry = [](uint32_t key, int id) { return (unsigned long long)key << 32 | (0xffffffffu - (uint32_t)id); };
+  each([&](float x, int) { atomicAdd(&hist[part(x)], 1); });
+  __syncthreads();
+  {
+    constexpr int B = kTopBins / NT;
+    int c[B], sum = 0, tot;
+#pragma unroll
+    for (int j = 0; j < B; ++j) sum += c[j] = hist[B * tid + j];
+    int above = block_excl_scan<NT>(sum, wt, tot);
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+      if (above < k && above + c[j] >= k) sh_bin = B * tid + j, sh_above = above;
+      above += c[j];
     }
-    __syncthreads();
-    if (tid == 0) {
-      int r = rem, b = 255;
-      for (; b > 0; --b) {
-        if (hist[b] >= r) break;
-        r -= hist[b];
-      }
-      sh_bin = b;
-      sh_rem = r;
-    }
-    __syncthreads();
-    prefix |= (uint32_t)sh_bin << shift;
-    mask |= 0xffu << shift;
-    rem = sh_rem;
-    __syncthreads();
   }
-  // prefix = key of the k-th largest; take every key > prefix and the first `rem` (by index) equal to it
-  int base = 0, eq_base = 0;
-  for (int c = 0; c < n; c += 1024) {
-    const int i = c + tid;
-    uint32_t key = 0;
-    if (i < n) key = order_key(row[i]);
-    const int gt = i < n && key > prefix, eq = i < n && key == prefix;
-    int eq_tot, sel_tot;
-    const int eq_rank = eq_base + block_excl_scan(eq, wt, eq_tot);
-    const int sel = gt || (eq && eq_rank < rem);
-    const int p = base + block_excl_scan(sel, wt, sel_tot);
-    if (sel && p < k) oi[p] = i;
-    base += sel_tot;
-    eq_base += eq_tot;
+  __syncthreads();
+  const int bin = sh_bin;
+  each([&](float x, int i) {
+    if (part(x) == bin) {
+      const int at = atomicAdd(&sh_n, 1);
+      if (at < kTopList) list[at] = entry(order_key(x), i);
+    }
+  });
+  __syncthreads();
+  const int m = sh_n, rem = k - sh_above;     // the rem-th largest of the list is the last selected
+  if (m <= kTopList) {
+    for (int i = tid; i < m; i += NT) {
+      const unsigned long long e = list[i];
+      int larger = 0;
+      for (int j = 0; j < m; ++j) larger += list[j] > e;
+      if (larger == rem - 1) sh_last = e;
+    }
+  } else {
+    uint32_t prefix = 0, mask = 0;
+    int left = k;  // how many still to take among entries matching the prefix
+    for (int shift = 24; shift >= 0; shift -= 8) {
+      __syncthreads();
+      for (int i = tid; i < 256; i += NT) hist[i] = 0;
+      __syncthreads();
+      each([&](float x, int) {
+        const uint32_t key = order_key(x);
+        if ((key & mask) == prefix) atomicAdd(&hist[255 - ((key >> shift) & 0xff)], 1);
+      });
+      __syncthreads();
+      int tot;
+      const int c = tid < 256 ? hist[tid] : 0, above = block_excl_scan<NT>(c, wt, tot);
+      if (above < left && above + c >= left) sh_bin = 255 - tid, sh_above = above;
+      __syncthreads();
+      prefix |= (uint32_t)sh_bin << shift;
+      mask |= 0xffu << shift;
+      left -= sh_above;
+    }
+    // of the entries equal to the k-th key the first `left` by index: the warp that holds the last of them names it
+    int eq = 0, tot;
+    each([&](float x, int) { eq += order_key(x) == prefix; });
+    eq = __reduce_add_sync(0xffffffffu, eq);
+    int before = block_excl_scan<NT>(lane == 0 ? eq : 0, wt, tot);
+    before = __shfl_sync(0xffffffffu, before, 0);
+    if (before < left && before + eq >= left) {
+      each4([&](const float4& x, int i) {
+        const float v[4] = {x.x, x.y, x.z, x.w};
+        unsigned bits = 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) bits |= (unsigned)(i + c < n && order_key(v[c]) == prefix) << c;
+        int rank = before, here = 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const unsigned all = __ballot_sync(0xffffffffu, bits >> c & 1);
+          rank += __popc(all & ((1u << lane) - 1)), here += __popc(all);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (bits >> c & 1) {
+            if (++rank == left) sh_last = entry(prefix, i + c);
+          }
+        before += here;
+      });
+    }
+  }
+  __syncthreads();
+  const unsigned long long last = sh_last;
+  int mine = 0, tot;
+  each([&](float x, int i) { mine += entry(order_key(x), i) >= last; });
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  int p = block_excl_scan<NT>(lane == 0 ? mine : 0, wt, tot);
+  p = __shfl_sync(0xffffffffu, p, 0);
+  if (mine > 0) {
+    each4([&](const float4& x, int i) {
+      const float v[4] = {x.x, x.y, x.z, x.w};
+      unsigned bits = 0;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) bits |= (unsigned)(i + c < n && entry(order_key(v[c]), i + c) >= last) << c;
+      int at = p;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const unsigned all = __ballot_sync(0xffffffffu, bits >> c & 1);
+        at += __popc(all & ((1u << lane) - 1)), p += __popc(all);
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (bits >> c & 1) {
+          if (at < k) oi[at] = i + c;
+          ++at;
+        }
+    });
   }
   if (tid == 0) out_len[t] = k;
 }
@@ -196,7 +324,13 @@ DSV4_API int dsv4_indexer_logits(const void* qc, const float* wf, const void* kv
 DSV4_API int dsv4_topk(const float* logits, int width, const int* pos, int* idx, int* out_len, int t, int k,
                        cudaStream_t st) {
   if (t <= 0) return 0;
-  dsv4_launch(topk_kernel, t, 1024, 0, st, logits, width, pos, idx, out_len, k);
+  // 16 or 32 entries a thread in registers
+  if (width <= 512 * 16)
+    dsv4_launch(topk_kernel<512, 4>, t, 512, 0, st, logits, width, pos, idx, out_len, k);
+  else if (width <= 1024 * 32)
+    dsv4_launch(topk_kernel<1024, 8>, t, 1024, 0, st, logits, width, pos, idx, out_len, k);
+  else
+    dsv4_launch(topk_kernel<1024, 0>, t, 1024, 0, st, logits, width, pos, idx, out_len, k);
   return (int)cudaGetLastError();
 }
 
