@@ -224,13 +224,14 @@ def indexer_select(qc, wf, vals, scales, fb, ps: int, k: int):
 def attention(q, fb, swa_cache, swa_map, comp_cache, ratio: int, topk_idx, topk_len, sink, scale, ps: int,
               window: int, out_rope=None):
     """``out_rope``: also rotate the last ``rotary_dim`` dims of every output row by minus its position (fused into
-    the kernel's epilogue on CUDA, :func:`rope_tail` with ``inverse=True`` on the oracle path)."""
+    the kernel's epilogue on CUDA, :func:`rope_tail` with ``inverse=True`` on the oracle path).
+    ``topk_idx`` [T, k], ``topk_len`` [T]: the 4:1 entries to attend; None: all that a token's position covers."""
     if q.is_cuda:
         return _cu().attention(q, fb, swa_cache, swa_map, comp_cache, ratio, topk_idx, topk_len, sink, scale, ps,
                                window, out_rope)
     srows = swa_rows(fb, swa_map, ps, window)
     crows = None
-    if ratio == 4:
+    if ratio == 4 and topk_idx is not None:
         idx = torch.where((topk_len > 0)[:, None], topk_idx, torch.full_like(topk_idx, -1))
         crows = comp_rows_from_idx(fb, idx, ps, 4)
     elif ratio:

@@ -21,6 +21,7 @@
 //   M = max_s m_s,  L = sum_s l_s e^(m_s - M),  o = sum_s acc_s e^(m_s - M) / L
 // -- and runs the usual epilogue.  The sink belongs to split 0.  The reference's decode kernel splits the same way
 // (python/minisgl/kernel/triton/deepseek_v4.py:1645, :2002-2050, up to 16 splits).
+#include "attention.cuh"
 #include "common.cuh"
 #include "rope.cuh"
 
@@ -53,34 +54,6 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-
-struct AttnArgs {
-  const __nv_bfloat16* q;
-  __nv_bfloat16* o;
-  const int* slots;
-  const int* pos;
-  const int* page_table;
-  int ld_pt;
-  const __nv_bfloat16* swa;
-  const int* swa_map;
-  const __nv_bfloat16* comp;
-  const int* topk_idx;
-  const int* topk_len;
-  int topk_width;
-  int mode;   // 0: window only, 1: compressed entries from topk_idx, 2: all compressed entries
-  int ratio;
-  const float* sink;
-  float scale;
-  int ps;
-  int window;
-  const int* num_valid;
-  int out_rope;   // != 0: rotate the last rp.rotary_dim dims of every output head row by -position (the inverse
-  RopeParams rp;  //       RoPE the output projection expects), on the bf16-rounded values, in the epilogue
-  int nsplit;        // CTAs per token (grid.y); > 1 needs the three buffers below
-  float* part_acc;   // [t][nsplit][HL][512] unnormalised accumulators
-  float* part_ml;    // [t][nsplit][HL][2]   running max and sum
-  int* counters;     // [t] zero between launches
-};
 
 // row of 512 bf16 = 64 chunks of 16 B; chunk c of row r is stored at chunk (c ^ (r & 7))
 __device__ __forceinline__ int swz_row(int r, int c) { return (c & ~7) | ((c ^ r) & 7); }
@@ -431,7 +404,7 @@ DSV4_API int dsv4_sparse_attention(const void* q, void* o, const int* slots, con
   if (t <= 0) return 0;
   if (d != D) return 300;
   if (nsplit < 1) nsplit = 1;
-  if (nsplit > 1 && (!part_acc || !part_ml || !counters)) return 305;
+  if (nsplit > 1 && (!part_acc || !part_ml || (!counters && heads != 64))) return 305;
   if (out_rope && (rp.rotary_dim <= 0 || rp.rotary_dim > 128 || rp.rotary_dim % 8)) return 303;
   AttnArgs a{(const __nv_bfloat16*)q, (__nv_bfloat16*)o, slots, pos, page_table, ld_pt, (const __nv_bfloat16*)swa,
              swa_map, (const __nv_bfloat16*)comp, topk_idx, topk_len, topk_width, mode, ratio, sink, scale, ps,
@@ -440,7 +413,7 @@ DSV4_API int dsv4_sparse_attention(const void* q, void* o, const int* slots, con
     case 8: return launch_attn<8>(a, t, st);
     case 16: return launch_attn<16>(a, t, st);
     case 32: return launch_attn<32>(a, t, st);
-    case 64: return launch_attn<64>(a, t, st);
+    case 64: return launch_attn_mma(a, t, st);
     default: return 302;
   }
 }

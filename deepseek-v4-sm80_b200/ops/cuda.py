@@ -318,10 +318,14 @@ _ATTN_COUNTERS = {}
 def attention_splits(t: int, heads: int, mode: int, ratio: int, topk_width: int, window: int, max_context: int,
                      prefill: bool, sms: int) -> int:
     """CTAs per token.  Splitting pays when the tokens alone leave SMs idle and a token has many key tiles (decode of
-    a few long sequences); a batch that fills the GPU, and every prefill chunk, runs one CTA per token."""
-    if prefill or t <= 0:
+    a few long sequences)."""
+    if t <= 0:
         return 1
     keys = window + (topk_width if mode == 1 else (max_context // ratio if mode == 2 else 0))
+    if heads == 64:                         # csrc/attention_mma.cu: 128 keys per tile, splits merged by a kernel of their own
+        return int(max(1, min(sms // t, -(-keys // 128), 32)))
+    if prefill:                             # one CTA per token
+        return 1
     kt = 64 if heads <= 16 else 32          # keys per tile of the kernel's configuration
     ntiles = -(-keys // kt)
     return int(max(1, min(sms // t, -(-ntiles // 2), 32)))
@@ -332,10 +336,11 @@ def attention_splits(t: int, heads: int, mode: int, ratio: int, topk_width: int,
 def attention(q, fb, swa_cache, swa_map, comp_cache, ratio: int, topk_idx, topk_len, sink, scale, ps: int,
               window: int, out_rope=None, nsplit: int = 0):
     """out_rope: RopeSpec whose inverse rotation the kernel applies to the tail of every output row.
-    nsplit: CTAs per token (0: chosen by :func:`attention_splits`)."""
+    nsplit: CTAs per token (0: chosen by :func:`attention_splits`).
+    topk_idx: the 4:1 entries to attend; None: all that the token's position covers."""
     t, h, d = q.shape
     o = torch.empty_like(q)
-    mode = 1 if ratio == 4 else (2 if ratio else 0)
+    mode = 0 if not ratio else 1 if ratio == 4 and topk_idx is not None else 2
     pt = fb.page_table
     if nsplit <= 0:
         nsplit = attention_splits(t, h, mode, ratio, topk_idx.shape[1] if mode == 1 else 0, window,
@@ -344,11 +349,12 @@ def attention(q, fb, swa_cache, swa_map, comp_cache, ratio: int, topk_idx, topk_
     if nsplit > 1:
         acc = torch.empty(t, nsplit, h, d, dtype=torch.float32, device=q.device)
         ml = torch.empty(t, nsplit, h, 2, dtype=torch.float32, device=q.device)
-        key = q.device.index or 0
-        cnt = _ATTN_COUNTERS.get(key)
-        if cnt is None or cnt.shape[0] < t:
-            cnt = torch.zeros(max(t, 4096), dtype=torch.int32, device=q.device)
-            _ATTN_COUNTERS[key] = cnt
+        if h != 64:
+            key = q.device.index or 0
+            cnt = _ATTN_COUNTERS.get(key)
+            if cnt is None or cnt.shape[0] < t:
+                cnt = torch.zeros(max(t, 4096), dtype=torch.int32, device=q.device)
+                _ATTN_COUNTERS[key] = cnt
     nv.call("sparse_attention", nv.ptr(q), nv.ptr(o), _i32(fb.slots), _i32(fb.positions), _i32(pt), I(pt.stride(0)),
             nv.ptr(swa_cache), _i32(swa_map), nv.ptr(comp_cache if mode else None),
             nv.ptr(topk_idx if mode == 1 else None), nv.ptr(topk_len if mode == 1 else None),
