@@ -278,47 +278,55 @@ __global__ void indexer_kv_store_kernel(const float* __restrict__ pooled, const 
 }
 
 // ------------------------------------------------------------------ indexer query (D = 128), one warp per (token, head)
-__global__ void indexer_q_encode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ wts,
-                                        const int* __restrict__ pos, RopeParams rp, float fold,
-                                        uint8_t* __restrict__ codes, float* __restrict__ wout, int heads, int rows) {
+// A warp takes eight heads of a token: their loads are in flight together, and the angles, which they share, are computed once, one
+// pair a lane.  4 096 tokens of 64 heads: 45 us (103 MB), 122 us with a warp per head.
+__global__ void __launch_bounds__(256) indexer_q_encode_kernel(const __nv_bfloat16* __restrict__ q,
+                                                               const __nv_bfloat16* __restrict__ wts, const int* __restrict__ pos,
+                                                               RopeParams rp, float fold, uint8_t* __restrict__ codes,
+                                                               float* __restrict__ wout, int heads, int t_rows) {
   pdl_entry();
-  constexpr int D = 128;
-  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  const int tok = row / heads;
-  float v[4];
-  {
-    const uint2 u = *reinterpret_cast<const uint2*>(q + (size_t)row * D + lane * 4);
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
-    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+  constexpr int D = 128, R = 8;
+  const int lane = threadIdx.x & 31, groups = (heads + R - 1) / R;
+  const int unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, tok = unit / groups, first = unit % groups * R;
+  if (tok >= t_rows) return;
+  const int n = min(R, heads - first), row0 = tok * heads + first;
+  uint2 u[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    u[r] = r < n ? *reinterpret_cast<const uint2*>(q + (size_t)(row0 + r) * D + lane * 4) : make_uint2(0, 0);
+  const float w = lane < n ? bf2f(wts[row0 + lane]) : 0.f;
+  float cs, sn;
+  rope_cos_sin(rp, (float)pos[tok], lane, 0, cs, sn);
+  const float c0 = __shfl_sync(0xffffffffu, cs, 2 * lane & 31), s0 = __shfl_sync(0xffffffffu, sn, 2 * lane & 31);
+  const float c1 = __shfl_sync(0xffffffffu, cs, (2 * lane + 1) & 31), s1 = __shfl_sync(0xffffffffu, sn, (2 * lane + 1) & 31);
+  float mine = 0.f;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (r >= n) break;
+    float v[4];
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[r].x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[r].y));
     v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
-  }
-  const int tail = D - rp.rotary_dim;
-  if (lane * 4 >= tail) {
-    const float pp = (float)pos[tok];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      float c, s;
-      rope_cos_sin(rp, pp, (lane * 4 - tail) / 2 + i, 0, c, s);
-      const float a = v[2 * i], b = v[2 * i + 1];
-      v[2 * i] = a * c - b * s;
-      v[2 * i + 1] = a * s + b * c;
+    if (lane >= 16) {     // dims 64 + 4 (lane - 16): pairs 2 lane - 32 and the next
+      v[0] = a.x * c0 - a.y * s0, v[1] = a.x * s0 + a.y * c0;
+      v[2] = b.x * c1 - b.y * s1, v[3] = b.x * s1 + b.y * c1;
     }
-  }
-  float amax = 0.f;
+    float amax = 0.f;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    v[i] = bf2f(f2bf(v[i]));
-    amax = fmaxf(amax, fabsf(v[i]));
-  }
-  amax = warp_max(amax);
-  const float sc = pow2_ceil_scale_c(amax), inv = 1.f / sc;
-  uint8_t o[4];
+    for (int i = 0; i < 4; ++i) {
+      v[i] = bf2f(f2bf(v[i]));
+      amax = fmaxf(amax, fabsf(v[i]));
+    }
+    amax = warp_max(amax);
+    const float sc = pow2_ceil_scale_c(amax), inv = 1.f / sc;
+    uint32_t o = 0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    o[i] = (uint8_t)__nv_cvt_float_to_fp8(fminf(fmaxf(v[i] * inv, -448.f), 448.f), __NV_SATFINITE, __NV_E4M3);
-  *reinterpret_cast<uint32_t*>(codes + (size_t)row * D + lane * 4) = *reinterpret_cast<uint32_t*>(o);
-  if (lane == 0) wout[row] = bf2f(wts[row]) * sc * fold;
+    for (int i = 0; i < 4; ++i)
+      o |= (uint32_t)__nv_cvt_float_to_fp8(fminf(fmaxf(v[i] * inv, -448.f), 448.f), __NV_SATFINITE, __NV_E4M3) << (8 * i);
+    *reinterpret_cast<uint32_t*>(codes + (size_t)(row0 + r) * D + lane * 4) = o;
+    if (lane == r) mine = sc;
+  }
+  if (lane < n) wout[row0 + lane] = w * mine * fold;
 }
 
 }  // namespace
@@ -365,8 +373,8 @@ DSV4_API int dsv4_indexer_q_encode(const void* q, const void* wts, const int* po
                                    void* codes, float* wout, int t, int heads, int d, cudaStream_t st) {
   if (t <= 0) return 0;
   if (d != 128 || rp.rotary_dim != 64) return 142;
-  const int rows = t * heads;
-  dsv4_launch(indexer_q_encode_kernel, (rows * 32 + 255) / 256, 256, 0, st, (const __nv_bfloat16*)q, (const __nv_bfloat16*)wts,
-                                                                  pos, rp, fold, (uint8_t*)codes, wout, heads, rows);
+  const int warps = t * ((heads + 7) / 8);
+  dsv4_launch(indexer_q_encode_kernel, (warps + 7) / 8, 256, 0, st, (const __nv_bfloat16*)q, (const __nv_bfloat16*)wts, pos, rp, fold,
+              (uint8_t*)codes, wout, heads, t);
   return (int)cudaGetLastError();
 }
