@@ -12,7 +12,7 @@
 //
 // A CTA owns one token group and a stride of the request's 128-key blocks.  Warp 0 walks the page table and feeds a
 // ring of key tiles by TMA (a page's compressed rows are contiguous, so a tile is 128 / rows-per-box box copies),
-// warp 1 issues the MMAs into one of two accumulators, warps 2-5 are the epilogue (one TMEM lane quarter each).
+// warp 1 issues the MMAs into one of two accumulators, the others are the epilogue (one TMEM lane quarter each).
 // Tokens of one group that belong to different requests (decode batches, request boundaries inside a prefill chunk)
 // are handled as separate passes over their own keys with N = 64.  Every wait is bounded.
 #include "common.cuh"
@@ -49,7 +49,10 @@ inline int idx_smem_bytes(int tg, int stages) { return stages * kATile + tg * kQ
 
 constexpr int kSmemBytes = SA * kATile + TGMAX * kQTile + TGMAX * HEADS * 4 + 256 + 1024;
 
-__global__ void __launch_bounds__(192, 1)
+// EW epilogue warps: 4, or for groups of several tokens 8, two to a quarter of the lanes, each with every other token.  A warp adds two
+// tokens' heads side by side: one token's sum is a chain of 64 additions, whose order fixes the result.
+template <int EW>
+__global__ void __launch_bounds__(64 + 32 * EW, EW == 4 ? 3 : 1)
 indexer_logits_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ,
                           const IdxArgs a) {
   extern __shared__ uint8_t ix_raw[];
@@ -74,7 +77,7 @@ indexer_logits_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
-    for (int i = 0; i < 2; ++i) mbar_init(&tfull[i], 1), mbar_init(&tempty[i], 128);
+    for (int i = 0; i < 2; ++i) mbar_init(&tfull[i], 1), mbar_init(&tempty[i], 32 * EW);
     mbar_init(qfull, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -196,10 +199,10 @@ indexer_logits_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_
     }
   } else {
     // ---------------- epilogue: warp w owns TMEM lanes (w % 4) * 32 .. + 31, i.e. 32 keys of every tile
-    const int q = warp & 3;
+    const int q = warp & 3, side = (warp - 2) >> 2;      // side: first token of a pass that this warp adds
     const int key_in_tile = q * 32 + lane;
-    for (int i = threadIdx.x - 64; i < ng * HEADS; i += 128) wfs[i] = a.wf[(size_t)t0 * HEADS + i];
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    for (int i = threadIdx.x - 64; i < ng * HEADS; i += 32 * EW) wfs[i] = a.wf[(size_t)t0 * HEADS + i];
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory");
     int it = 0;
     bool ok = true;
     for (int p = 0; p < npass && ok; ++p) {
@@ -220,19 +223,48 @@ indexer_logits_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_
         }
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + b * (a.tg * HEADS);
-        for (int c = 0; c < p_cnt[p]; ++c) {
+        constexpr int kStep = EW / 4;
+        for (int c = side; c < p_cnt[p]; c += 2 * kStep) {
           const int g = p_first[p] + c;
-          const float* w = wfs + g * HEADS;
-          float acc = 0.f;
+          const bool two = c + kStep < p_cnt[p];
+          const float* w0 = wfs + g * HEADS;
+          const float* w1 = two ? w0 + kStep * HEADS : w0;
+          float acc0 = 0.f, acc1 = 0.f;
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
-            uint32_t r[32];
-            tmem_ld_32x32(taddr + c * HEADS + half * 32, r);
+            uint32_t r0[32], r1[32];
+            tmem_ld_32x32(taddr + c * HEADS + half * 32, r0);
+            if (two) tmem_ld_32x32(taddr + (c + kStep) * HEADS + half * 32, r1);
             tmem_ld_wait();
+            if (two) {
 #pragma unroll
-            for (int h = 0; h < 32; ++h) acc = fmaf(fmaxf(__uint_as_float(r[h]), 0.f), w[half * 32 + h], acc);
+              for (int h = 0; h < 32; h += 4) {
+                const float4 a0 = *reinterpret_cast<const float4*>(w0 + half * 32 + h);
+                const float4 a1 = *reinterpret_cast<const float4*>(w1 + half * 32 + h);
+                acc0 = fmaf(fmaxf(__uint_as_float(r0[h]), 0.f), a0.x, acc0);
+                acc1 = fmaf(fmaxf(__uint_as_float(r1[h]), 0.f), a1.x, acc1);
+                acc0 = fmaf(fmaxf(__uint_as_float(r0[h + 1]), 0.f), a0.y, acc0);
+                acc1 = fmaf(fmaxf(__uint_as_float(r1[h + 1]), 0.f), a1.y, acc1);
+                acc0 = fmaf(fmaxf(__uint_as_float(r0[h + 2]), 0.f), a0.z, acc0);
+                acc1 = fmaf(fmaxf(__uint_as_float(r1[h + 2]), 0.f), a1.z, acc1);
+                acc0 = fmaf(fmaxf(__uint_as_float(r0[h + 3]), 0.f), a0.w, acc0);
+                acc1 = fmaf(fmaxf(__uint_as_float(r1[h + 3]), 0.f), a1.w, acc1);
+              }
+            } else {
+#pragma unroll
+              for (int h = 0; h < 32; h += 4) {
+                const float4 a0 = *reinterpret_cast<const float4*>(w0 + half * 32 + h);
+                acc0 = fmaf(fmaxf(__uint_as_float(r0[h]), 0.f), a0.x, acc0);
+                acc0 = fmaf(fmaxf(__uint_as_float(r0[h + 1]), 0.f), a0.y, acc0);
+                acc0 = fmaf(fmaxf(__uint_as_float(r0[h + 2]), 0.f), a0.z, acc0);
+                acc0 = fmaf(fmaxf(__uint_as_float(r0[h + 3]), 0.f), a0.w, acc0);
+              }
+            }
           }
-          if (j < a.width) a.logits[(size_t)(t0 + g) * a.width + j] = j < n_tok[g] ? acc * ks : -INFINITY;
+          if (j < a.width) {
+            a.logits[(size_t)(t0 + g) * a.width + j] = j < n_tok[g] ? acc0 * ks : -INFINITY;
+            if (two) a.logits[(size_t)(t0 + g + kStep) * a.width + j] = j < n_tok[g + kStep] ? acc1 * ks : -INFINITY;
+          }
         }
         tc_fence_before();
         mbar_arrive(&tempty[b]);
@@ -270,8 +302,8 @@ DSV4_API int dsv4_indexer_logits_mma(const void* qc, const float* wf, const void
   if (dsv4_make_tmap_2d(&tmQ, qc, 0, DI, (uint64_t)t * HEADS, DI, DI, HEADS, 3)) return 475;
   static bool set = false;
   if (!set) {
-    if (cudaFuncSetAttribute(indexer_logits_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(indexer_logits_mma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess ||
+        cudaFuncSetAttribute(indexer_logits_mma_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
       return 476;
     set = true;
   }
@@ -280,6 +312,9 @@ DSV4_API int dsv4_indexer_logits_mma(const void* qc, const float* wf, const void
   IdxArgs a{wf, kscale, slots, pos, page_table, ld_pt, ps, logits, width, t, tg, box_rows, stages, tmem_cols};
   const int groups = (t + tg - 1) / tg;
   if (nsplit < 1) nsplit = 1;
-  dsv4_launch(indexer_logits_mma_kernel, dim3(nsplit, groups), 192, idx_smem_bytes(tg, stages), st, tmK, tmQ, a);
+  if (tg == 1)
+    dsv4_launch(indexer_logits_mma_kernel<4>, dim3(nsplit, groups), 192, idx_smem_bytes(tg, stages), st, tmK, tmQ, a);
+  else
+    dsv4_launch(indexer_logits_mma_kernel<8>, dim3(nsplit, groups), 320, idx_smem_bytes(tg, stages), st, tmK, tmQ, a);
   return (int)cudaGetLastError();
 }
