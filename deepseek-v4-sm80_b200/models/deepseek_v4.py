@@ -105,6 +105,9 @@ class DSV4Model:
             yq = O.fp8_quant(y)
         iw = None
         qkv = None
+        # a history of no more entries than are selected is attended whole: its queries and scores for a choice are not computed (the
+        # indexer's cache is written all the same, for later tokens)
+        choose = ratio == 4 and fb.max_context // 4 > cfg.index_topk
         if sp is not None:
             # the all-gather is fused into this GEMM's loads; everything else that reads y is issued behind it
             from ..ops.gemm import gemm_fp8_gated
@@ -113,8 +116,9 @@ class DSV4Model:
         if ratio:
             # compressor (and indexer cache) branch: depends only on y, meets the query chain at the selection
             with self._fork(y):
-                if ratio == 4:
+                if choose:
                     iw = O.gemm_bf16(y, w[p + "idx.weights_proj"])
+                if ratio == 4:
                     n1 = w[p + "comp.wkv_gate"].shape[0]
                     both = O.gemm_bf16(y, w[p + "comp_all.wkv_gate"], out_dtype=torch.float32)  # one GEMM, two slices
                     proj, proj_i = both[:, :n1], both[:, n1:]
@@ -135,12 +139,12 @@ class DSV4Model:
         q, kv = O.q_kv_norm_rope_store(q, kv, fb.positions, w[p + "kv_norm.weight"], cfg.rms_norm_eps, rope,
                                        kvv["swa"], fb.out_loc, self.pool.swa_map, ps, self.qat)
         topk_idx = topk_len = None
-        if ratio == 4:
+        if choose:
             iq = O.gemm_fp8(qlq[0], qlq[1], w[p + "idx.wq_b.weight"], w[p + "idx.wq_b.scale"])
             iq = iq.view(t, cfg.index_n_heads, cfg.index_head_dim)
         if ratio:
             self._join(y)
-        if ratio == 4:
+        if choose:
             qc, wf = O.indexer_q_encode(iq, iw, fb.positions, rope, cfg.index_head_dim ** -0.5,
                                         cfg.index_n_heads ** -0.5)
             topk_idx, topk_len = O.indexer_select(qc, wf, kvv["idx_vals"], kvv["idx_scale"], fb, ps, cfg.index_topk)
