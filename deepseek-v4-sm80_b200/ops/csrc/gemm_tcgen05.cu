@@ -639,6 +639,7 @@ DSV4_API int dsv4_gemm_set_weight_prefetch(int on) {
   g_weight_prefetch = on ? 1 : 0;
   return 0;
 }
+int dsv4_weight_prefetch() { return g_weight_prefetch; }
 
 // Workspace floats needed for a split-K launch: tiles * splits * 128 * bn.
 DSV4_API long long dsv4_gemm_splitk_ws_elems(int M, int N, int bn, int batches, int splits) {

@@ -142,6 +142,10 @@ def gemm_bf16(x, w, out=None, out_dtype=torch.bfloat16, accumulate=False, bn=0, 
                 I(o2.stride(0)), I(1 if out.dtype == torch.float32 else 0), I(1 if accumulate else 0), I(ACTS[act]), F(0.0), I(1),
                 I(NUM_SMS_HINT))
         return out
+    if bn == 0 and splits == 0 and act is None and _few_rows(x2, w, m, k, 32):
+        nv.call("gemm_rows_bf16", nv.ptr(x2), nv.ptr(w), nv.ptr(o2), I(m), I(n), I(k), I(x2.stride(0)), I(w.stride(0)),
+                I(o2.stride(0)), I(1 if out.dtype == torch.float32 else 0), I(1 if accumulate else 0), I(1))
+        return out
     bn, splits = pick_tiling(m, n, (k + 63) // 64, 1, False, bn, splits)
     ws, cnt = _ws(m, n, bn, 1, splits, x.device)
     nv.call("gemm_bf16", nv.ptr(x2), nv.ptr(w), nv.ptr(o2), I(m), I(n), I(k), I(x2.stride(0)), I(w.stride(0)),
@@ -169,6 +173,18 @@ def prefill_tiles(m: int, n: int, groups: int) -> int:
 def _many_rows(x2, w, m: int, n: int, k: int, groups: int) -> bool:
     """Whether the persistent kernel takes this bf16 projection."""
     return prefill_tiles(m, n, groups) >= PREFILL_MIN_TILES and _tma_ok(x2, w, k)
+
+
+# Rows up to which the kernel without tiles (csrc/gemm_rows.cu) is the faster one: its work grows by the eight rows, the tiled kernel's
+# does not up to 128.  The projections of an attention block take 87 us there at 24 rows, 102 at 30, and 95 in tiles.
+FEW_ROWS = 24
+
+
+def _few_rows(x2, w, m: int, k: int, whole: int) -> bool:
+    """Whether the kernel for a few rows takes this projection: K in multiples of `whole`, rows on 16 bytes."""
+    e = x2.element_size()
+    return (0 < m <= FEW_ROWS and k % whole == 0 and x2.stride(0) * e % 16 == 0 and w.stride(0) * e % 16 == 0
+            and x2.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 def linear(x, w, out=None, out_dtype=None, accumulate=False, act=None, limit=0.0):
@@ -270,6 +286,10 @@ def gemm_bf16_grouped(x, w, groups: int, out=None):
         nv.call("gemm_prefill", nv.ptr(x), nv.ptr(w), nv.ptr(out), I(t), I(n), I(k), I(x.stride(0)), I(w.stride(0)),
                 I(out.stride(0)), I(0), I(0), I(0), F(0.0), I(groups), I(NUM_SMS_HINT))
         return out
+    if _few_rows(x, w, t, k, 32):
+        nv.call("gemm_rows_bf16", nv.ptr(x), nv.ptr(w), nv.ptr(out), I(t), I(n), I(k), I(x.stride(0)), I(w.stride(0)), I(out.stride(0)),
+                I(1 if out.dtype == torch.float32 else 0), I(0), I(groups))
+        return out
     bn, splits = pick_tiling(t, n, (k + 63) // 64, groups, False, 0, 0)
     ws, cnt = _ws(t, n, bn, groups, splits, x.device)
     nv.call("gemm_bf16", nv.ptr(x), nv.ptr(w), nv.ptr(out), I(t), I(n), I(k), I(x.stride(0)), I(w.stride(0)),
@@ -302,6 +322,10 @@ def gemm_fp8(xq, sx, wq, sw, out=None, out_dtype=torch.bfloat16, accumulate=Fals
         nv.call("gemm_prefill_fp8", nv.ptr(x2), nv.ptr(wq), nv.ptr(o2), nv.ptr(s2), nv.ptr(sw), I(m), I(n), I(k), I(x2.stride(0)),
                 I(wq.stride(0)), I(o2.stride(0)), I(1 if out.dtype == torch.float32 else 0), I(1 if accumulate else 0),
                 I(NUM_SMS_HINT))
+        return out
+    if bn == 0 and splits == 0 and _few_rows(x2, wq, m, k, 128):
+        nv.call("gemm_rows_fp8", nv.ptr(x2), nv.ptr(wq), nv.ptr(o2), nv.ptr(s2), nv.ptr(sw), I(m), I(n), I(k), I(x2.stride(0)),
+                I(wq.stride(0)), I(o2.stride(0)), I(1 if out.dtype == torch.float32 else 0), I(1 if accumulate else 0))
         return out
     bn, splits = pick_tiling(m, n, k // 128, 1, True, bn, splits)
     ws, cnt = _ws(m, n, bn, 1, splits, xq.device)
