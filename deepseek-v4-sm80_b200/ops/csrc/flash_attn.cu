@@ -13,6 +13,8 @@
 //   warp 0      TMA producer: Q once, then K and V^T tiles through two-stage rings
 //   warp 1      tcgen05.mma issuer:  S_t = Q_t K^T,  O_t += P_t V  (P_t is read from tensor memory)
 //   warps 2-5   softmax of tile 0, warps 6-9 of tile 1: one thread per row; P_t overwrites S_t in place as bf16
+// The softmax warps' instructions bound it: multiplications and additions are issued two at a time (8 192 tokens of 16 heads of 128
+// with capped scores 384 us, 446 us one at a time).
 // Tensor memory: S0 | S1 | O0 | O1, 128 columns each.  O stays there; it is rescaled only when a row's maximum has grown by
 // more than 2^8 since the last time (the sums stay far from overflow, the quotient does not depend on it).
 #include "mma16.cuh"
@@ -235,9 +237,12 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           float* x = s + c;
           if (small) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float y = x[j] * x[j];
-              x[j] *= fmaf(fmaf(fmaf(a.p3, y, a.p2), y, a.p1), y, a.p0);
+            for (int j = 0; j < 32; j += 2) {
+              const float2 v = make_float2(x[j], x[j + 1]), y = mul_x2(v, v);
+              float2 f = fma_x2(make_float2(a.p3, a.p3), y, make_float2(a.p2, a.p2));
+              f = fma_x2(f, y, make_float2(a.p1, a.p1));
+              f = mul_x2(v, fma_x2(f, y, make_float2(a.p0, a.p0)));
+              x[j] = f.x, x[j + 1] = f.y;
             }
           } else {
 #pragma unroll
@@ -307,20 +312,21 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           }
         }
       }
-      float sum0 = 0.f, sum1 = 0.f;
+      float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t pk[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          const float p0 = ex2(fmaf(s[c * 32 + 2 * j], sc, -m)), p1 = ex2(fmaf(s[c * 32 + 2 * j + 1], sc, -m));
-          sum0 += p0, sum1 += p1;
-          const __nv_bfloat162 p = __floats2bfloat162_rn(p0, p1);
+          const float2 e = fma_x2(make_float2(s[c * 32 + 2 * j], s[c * 32 + 2 * j + 1]), make_float2(sc, sc), make_float2(-m, -m));
+          const float2 w = make_float2(ex2(e.x), ex2(e.y));
+          sum = add_x2(sum, w);
+          const __nv_bfloat162 p = __floats2bfloat162_rn(w.x, w.y);
           pk[j] = *reinterpret_cast<const uint32_t*>(&p);
         }
         tmem_st_32x16(sp + c * 16, pk);
       }
-      l += sum0 + sum1;
+      l += sum.x + sum.y;
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(&b->p_ready[t]);
