@@ -36,6 +36,7 @@ struct PlanHeader {
 // scoring 3: the bias belongs to the logits, the k largest z = score + bias are selected and weighted with the softmax
 // over the selected logits only (p = e^(z - max z); the largest is always selected, so the sum is at least 1).
 // scoring 2: p is the softmax over all logits; scoring 4: the same, and the weights are p * scaling as they are.
+template <int MAXPER>     // experts per lane at most
 __global__ void moe_topk_kernel(const float* __restrict__ scores, const float* __restrict__ bias,
                                 const int* __restrict__ tid2eid, const int* __restrict__ token_ids,
                                 const int* __restrict__ num_valid, int* __restrict__ idx, float* __restrict__ wts,
@@ -50,7 +51,6 @@ __global__ void moe_topk_kernel(const float* __restrict__ scores, const float* _
     if (lane < k) idx[row * k + lane] = -1, wts[row * k + lane] = 0.f;
     return;
   }
-  constexpr int MAXPER = 16;  // e <= 512
   float p[MAXPER], sel[MAXPER];
   const int per = (e + 31) / 32;
   float sc[MAXPER];
@@ -58,14 +58,20 @@ __global__ void moe_topk_kernel(const float* __restrict__ scores, const float* _
   for (int i = 0; i < MAXPER; ++i) sc[i] = 0.f;
   {
     const float* sp = scores + (size_t)row * e + lane;
-#pragma unroll 2
-    for (int q = 0; q < n_part; ++q) {
-      float tmp[MAXPER];
+    // eight splits in flight (a decode batch has about 18); they are added in order
+    constexpr int U = MAXPER <= 8 ? 8 : 4;
+    for (int q0 = 0; q0 < n_part; q0 += U) {
+      float tmp[U][MAXPER];
 #pragma unroll
-      for (int i = 0; i < MAXPER; ++i)
-        tmp[i] = (i < per && lane + i * 32 < e) ? __ldg(sp + (size_t)q * part_stride + i * 32) : 0.f;
+      for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int i = 0; i < MAXPER; ++i) sc[i] += tmp[i];
+        for (int i = 0; i < MAXPER; ++i)
+          tmp[u][i] = (q0 + u < n_part && i < per && lane + i * 32 < e) ? __ldg(sp + (size_t)(q0 + u) * part_stride + i * 32) : 0.f;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int i = 0; i < MAXPER; ++i)
+          if (q0 + u < n_part) sc[i] += tmp[u][i];
     }
   }
   float smax = -INFINITY;
@@ -162,57 +168,87 @@ __global__ void moe_topk_kernel(const float* __restrict__ scores, const float* _
 // ------------------------------------------------------------------ route planning (one CTA)
 // Local routes (expert in [base, base+e_local)) are grouped by expert; order inside a group is arbitrary
 // (every route row is computed independently and lands in its own output row, so results do not depend on it).
+// Bound by latency and, for many routes, by the scattered stores of an SM: every CTA counts all routes, and writes those of its own
+// range.  A route's rank within its expert is what the count returns, eight routes a thread are in flight, and the experts' first
+// positions come from a scan.  30 routes of 256 experts take 3.5 us (one thread adding up the experts and two dependent steps per
+// route: 17), 49 152 routes 16 us (91).
+constexpr int kPlanRange = 4096;    // routes per CTA from which on more CTAs share them, up to 16
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ idx, const float* __restrict__ wts,
                                                         int routes, int e_local, int base, int nt,
                                                         PlanHeader* __restrict__ hdr, int* __restrict__ tiles,
-                                                        int* __restrict__ sorted_route, int* __restrict__ route_pos,
+                                                        int* __restrict__ sorted_route, int* route_pos,
                                                         float* __restrict__ sorted_w) {
   pdl_entry();
   extern __shared__ int sm[];
   int* cnt = sm;                 // [e_local]
-  int* off = sm + e_local;       // [e_local + 1]
-  int* cur = off + e_local + 1;  // [e_local]
-  int* toff = cur + e_local;     // [e_local + 1]
-  for (int i = threadIdx.x; i < e_local; i += blockDim.x) cnt[i] = 0;
+  int* off = sm + e_local;       // [e_local]
+  __shared__ int wr[32], wt[32];
+  constexpr int U = 8;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int range = (routes + gridDim.x - 1) / gridDim.x, lo = min((int)blockIdx.x * range, routes), hi = min(lo + range, routes);
+  for (int i = tid; i < e_local; i += 1024) cnt[i] = 0;
   __syncthreads();
-  for (int r = threadIdx.x; r < routes; r += blockDim.x) {
-    const int e = idx[r] - base;
-    if (idx[r] >= 0 && e >= 0 && e < e_local) atomicAdd(&cnt[e], 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int a = 0, ta = 0;
-    for (int i = 0; i < e_local; ++i) {
-      off[i] = a;
-      toff[i] = ta;
-      a += cnt[i];
-      ta += (cnt[i] + nt - 1) / nt;
+  auto count = [&](int from, int to, bool own) {
+    for (int r0 = from + tid; r0 < to; r0 += 1024 * U) {
+      int id[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) id[u] = r0 + 1024 * u < to ? idx[r0 + 1024 * u] : -1;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int e = id[u] - base;
+        const int rank = id[u] >= 0 && e >= 0 && e < e_local ? atomicAdd(&cnt[e], 1) : -1;
+        if (own && r0 + 1024 * u < to) route_pos[r0 + 1024 * u] = rank;
+      }
     }
-    off[e_local] = a;
-    toff[e_local] = ta;
-    hdr->num_tiles = ta;
-    hdr->num_routes_local = a;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < e_local; i += blockDim.x) {
-    cur[i] = 0;
-    const int n = cnt[i];
-    for (int c = 0, ti = toff[i]; c < n; c += nt, ++ti) {
-      tiles[ti * 3 + 0] = i;
-      tiles[ti * 3 + 1] = off[i] + c;
-      tiles[ti * 3 + 2] = min(nt, n - c);
+    __syncthreads();
+  };
+  count(0, lo, false);
+  count(lo, hi, true);
+  count(hi, routes, false);
+  int r_sum = 0, t_sum = 0;      // routes and tiles of the experts before this round of 1 024
+  for (int i0 = 0; i0 < e_local; i0 += 1024) {
+    const int i = i0 + tid, n = i < e_local ? cnt[i] : 0, nti = (n + nt - 1) / nt;
+    int r = n, t = nti;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, r, o), y = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) r += x, t += y;
     }
+    if (lane == 31) wr[warp] = r, wt[warp] = t;
+    __syncthreads();
+    int rb = r_sum, tb = t_sum;
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) rb += wr[w], tb += wt[w];
+      r_sum += wr[w], t_sum += wt[w];
+    }
+    if (i < e_local) {
+      off[i] = rb + r - n;
+      if (blockIdx.x == 0)
+        for (int c = 0, ti = tb + t - nti; c < n; c += nt, ++ti) {
+          tiles[ti * 3 + 0] = i;
+          tiles[ti * 3 + 1] = rb + r - n + c;
+          tiles[ti * 3 + 2] = min(nt, n - c);
+        }
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  for (int r = threadIdx.x; r < routes; r += blockDim.x) {
-    const int e = idx[r] - base;
-    if (idx[r] >= 0 && e >= 0 && e < e_local) {
-      const int pos = off[e] + atomicAdd(&cur[e], 1);
+  if (blockIdx.x == 0 && tid == 0) hdr->num_tiles = t_sum, hdr->num_routes_local = r_sum;
+  for (int r0 = lo + tid; r0 < hi; r0 += 1024 * U) {
+    int id[U], rank[U];
+    float w[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = r0 + 1024 * u;
+      id[u] = rank[u] = -1, w[u] = 0.f;
+      if (r < hi) id[u] = idx[r], rank[u] = route_pos[r], w[u] = wts[r];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (rank[u] < 0) continue;
+      const int r = r0 + 1024 * u, pos = off[id[u] - base] + rank[u];
       sorted_route[pos] = r;
-      sorted_w[pos] = wts[r];
+      sorted_w[pos] = w[u];
       route_pos[r] = pos;
-    } else {
-      route_pos[r] = -1;
     }
   }
 }
@@ -824,8 +860,8 @@ DSV4_API int dsv4_moe_topk(const float* scores, const float* bias, const int* ti
   if (t <= 0) return 0;
   if (e > 512 || k > 32 || n_part < 1) return 210;
   // one warp per token, two warps per CTA: a decode batch of 128 tokens then covers 64 SMs instead of 16
-  dsv4_launch(moe_topk_kernel, (t * 32 + 63) / 64, 64, 0, st, scores, bias, tid2eid, token_ids, num_valid, idx, wts, t,
-              e, k, scaling, scoring, n_part, part_stride);
+  dsv4_launch(e <= 256 ? moe_topk_kernel<8> : moe_topk_kernel<16>, (t * 32 + 63) / 64, 64, 0, st, scores, bias, tid2eid, token_ids,
+              num_valid, idx, wts, t, e, k, scaling, scoring, n_part, part_stride);
   return (int)cudaGetLastError();
 }
 
@@ -837,8 +873,9 @@ DSV4_API int dsv4_moe_plan(const int* idx, const float* wts, int routes, int e_l
   int* sorted_route = tiles + 3 * max_tiles;
   int* route_pos = sorted_route + routes;
   float* sorted_w = reinterpret_cast<float*>(route_pos + routes);
-  const int smem = (4 * e_local + 2) * sizeof(int);
-  dsv4_launch(moe_plan_kernel, 1, 1024, smem, st, idx, wts, routes, e_local, base, nt, hdr, tiles, sorted_route, route_pos,
+  const int smem = 2 * e_local * sizeof(int);
+  const int ctas = routes <= kPlanRange ? 1 : routes >= 16 * kPlanRange ? 16 : (routes + kPlanRange - 1) / kPlanRange;
+  dsv4_launch(moe_plan_kernel, ctas, 1024, smem, st, idx, wts, routes, e_local, base, nt, hdr, tiles, sorted_route, route_pos,
                                          sorted_w);
   return (int)cudaGetLastError();
 }
