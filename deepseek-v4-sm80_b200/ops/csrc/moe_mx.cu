@@ -54,52 +54,53 @@ __device__ __forceinline__ void mx_block_exps(float amax, int& eh, int& el) {
   eh = min(max(ef - 7, 5), 253);
   el = eh - 5;
 }
-__device__ __forceinline__ float e4m3_to_float(uint32_t b) {
-  const __half_raw hr = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)b, __NV_E4M3);
-  return __half2float(*reinterpret_cast<const __half*>(&hr));
-}
-// x (a bf16 value held in fp32) -> (hi, lo) bytes under the block exponents
-__device__ __forceinline__ void mx_split(float x, int eh, int el, uint32_t& hi, uint32_t& lo) {
+// two bf16 values (held in fp32) -> two hi and two lo bytes under the block exponents
+__device__ __forceinline__ void mx_split2(float x0, float x1, int eh, int el, uint32_t& hi, uint32_t& lo) {
   const float inv_h = __uint_as_float((uint32_t)(254 - eh) << 23), s_h = __uint_as_float((uint32_t)eh << 23);
   const float inv_l = __uint_as_float((uint32_t)(254 - el) << 23);
-  hi = __nv_cvt_float_to_fp8(x * inv_h, __NV_SATFINITE, __NV_E4M3);
-  const float r = x - e4m3_to_float(hi) * s_h;
-  lo = __nv_cvt_float_to_fp8(r * inv_l, __NV_SATFINITE, __NV_E4M3);
+  const __nv_fp8x2_storage_t h = __nv_cvt_float2_to_fp8x2(make_float2(x0 * inv_h, x1 * inv_h), __NV_SATFINITE, __NV_E4M3);
+  const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(h, __NV_E4M3);
+  const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&hr));
+  hi = h;
+  lo = __nv_cvt_float2_to_fp8x2(make_float2((x0 - b.x * s_h) * inv_l, (x1 - b.y * s_h) * inv_l), __NV_SATFINITE, __NV_E4M3);
 }
 // byte offset of (row n, K block kb) inside a 512-byte scale block of 128 rows x 4 K blocks
 __device__ __forceinline__ int sf_offset(int n, int kb) { return (n & 31) * 16 + (n >> 5) * 4 + kb; }
 
-// xq[2 pos] = hi row, xq[2 pos + 1] = lo row of x[sorted_route[pos] / topk]; the block exponents go into the scale
-// block of the position's route tile: sf[tile][K / 128][512] at rows 2 n and 2 n + 1, n = pos - tile start.
+// xq[2 pos] = hi row, xq[2 pos + 1] = lo row of token t for every route of t, pos = route_pos[t * topk + k]; the block exponents go
+// into the scale block of the position's route tile: sf[tile][K / 128][512] at rows 2 n and 2 n + 1, n = pos - tile start.
+// A CTA per token: its row is read and split once, for all of its routes.  8 192 tokens of six routes: 133 us, 227 us with a CTA per
+// route.
+constexpr int kMaxTopk = 32;
 __global__ void __launch_bounds__(128) moe_mx_permute_kernel(const __nv_bfloat16* __restrict__ x,
                                                              uint8_t* __restrict__ xq, uint8_t* __restrict__ sf,
                                                              const MxPlanHeader* __restrict__ hdr,
                                                              const int* __restrict__ tiles,
-                                                             const int* __restrict__ sorted_route, int topk, int h,
+                                                             const int* __restrict__ route_pos, int topk, int h,
                                                              int routes, int max_tiles, int nt) {
   pdl_entry();
-  const int pos = blockIdx.x;
-  if (pos >= hdr->num_routes_local) return;
-  if (hdr->num_tiles < 1 || hdr->num_tiles > max_tiles || hdr->num_routes_local > routes) {  // a plan from other sizes
+  if (hdr->num_tiles < 0 || hdr->num_tiles > max_tiles || hdr->num_routes_local > routes) {  // a plan from other sizes
     if (threadIdx.x == 0) dsv4_set_error(DSV4_ERR_BAD_INDEX, 31, hdr->num_tiles);
     return;
   }
-  __shared__ int s_tile;
-  if (threadIdx.x == 0) {  // the last tile that starts at or before pos (tiles are in position order)
-    int lo = 0, hi = hdr->num_tiles - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (tiles[mid * 3 + 1] <= pos) lo = mid; else hi = mid - 1;
+  __shared__ int s_pos[kMaxTopk], s_tile[kMaxTopk], s_n[kMaxTopk];
+  const int tok = blockIdx.x;
+  if (threadIdx.x < topk) {
+    const int pos = route_pos[tok * topk + threadIdx.x];
+    int keep = -1, tile = 0, n = 0;
+    if (pos >= 0 && pos < hdr->num_routes_local) {
+      int lo = 0, hi = hdr->num_tiles - 1;   // the last tile that starts at or before pos (tiles are in position order)
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tiles[mid * 3 + 1] <= pos) lo = mid; else hi = mid - 1;
+      }
+      tile = lo, n = hi >= 0 ? pos - tiles[lo * 3 + 1] : -1;
+      if (n >= 0 && n < nt) keep = pos;
     }
-    s_tile = lo;
+    if (keep < 0 && pos != -1) dsv4_set_error(DSV4_ERR_BAD_INDEX, 32, pos);
+    s_pos[threadIdx.x] = keep, s_tile[threadIdx.x] = tile, s_n[threadIdx.x] = n;
   }
   __syncthreads();
-  const int ti = s_tile, n = pos - tiles[ti * 3 + 1];
-  const int tok = sorted_route[pos] / topk;
-  if (n < 0 || n >= nt || sorted_route[pos] < 0 || sorted_route[pos] >= routes) {
-    if (threadIdx.x == 0) dsv4_set_error(DSV4_ERR_BAD_INDEX, 32, pos);
-    return;
-  }
   const int nblk = h / 32, nchunks = h / 128;
   for (int blk = threadIdx.x; blk < nblk; blk += blockDim.x) {
     const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)tok * h + blk * 32);
@@ -114,19 +115,23 @@ __global__ void __launch_bounds__(128) moe_mx_permute_kernel(const __nv_bfloat16
     mx_block_exps(amax, eh, el);
     uint32_t wh[8] = {0, 0, 0, 0, 0, 0, 0, 0}, wl[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
+    for (int i = 0; i < 32; i += 2) {
       uint32_t hb, lb;
-      mx_split(f[i], eh, el, hb, lb);
+      mx_split2(f[i], f[i + 1], eh, el, hb, lb);
       wh[i >> 2] |= hb << (8 * (i & 3));
       wl[i >> 2] |= lb << (8 * (i & 3));
     }
-    uint4* dh = reinterpret_cast<uint4*>(xq + (size_t)(2 * pos) * h + blk * 32);
-    uint4* dl = reinterpret_cast<uint4*>(xq + (size_t)(2 * pos + 1) * h + blk * 32);
-    dh[0] = make_uint4(wh[0], wh[1], wh[2], wh[3]), dh[1] = make_uint4(wh[4], wh[5], wh[6], wh[7]);
-    dl[0] = make_uint4(wl[0], wl[1], wl[2], wl[3]), dl[1] = make_uint4(wl[4], wl[5], wl[6], wl[7]);
-    uint8_t* sb = sf + ((size_t)ti * nchunks + (blk >> 2)) * 512;
-    sb[sf_offset(2 * n, blk & 3)] = (uint8_t)eh;
-    sb[sf_offset(2 * n + 1, blk & 3)] = (uint8_t)el;
+    for (int k = 0; k < topk; ++k) {
+      const int pos = s_pos[k], n = s_n[k];
+      if (pos < 0) continue;
+      uint4* dh = reinterpret_cast<uint4*>(xq + (size_t)(2 * pos) * h + blk * 32);
+      uint4* dl = reinterpret_cast<uint4*>(xq + (size_t)(2 * pos + 1) * h + blk * 32);
+      dh[0] = make_uint4(wh[0], wh[1], wh[2], wh[3]), dh[1] = make_uint4(wh[4], wh[5], wh[6], wh[7]);
+      dl[0] = make_uint4(wl[0], wl[1], wl[2], wl[3]), dl[1] = make_uint4(wl[4], wl[5], wl[6], wl[7]);
+      uint8_t* sb = sf + ((size_t)s_tile[k] * nchunks + (blk >> 2)) * 512;
+      sb[sf_offset(2 * n, blk & 3)] = (uint8_t)eh;
+      sb[sf_offset(2 * n + 1, blk & 3)] = (uint8_t)el;
+    }
   }
 }
 
@@ -171,7 +176,10 @@ moe_mx_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                    float limit, int e_local, int routes, int max_tiles) {
   using S = MxSmem<MODE, NT>;
   constexpr int kStages = S::kStages, kChunks = S::kChunks, kAccSets = S::kAccSets;
-  constexpr uint32_t kIdesc = umma_idesc_mx(128, 2 * NT, 5, 0);  // e2m1 x e4m3, ue8m0 scales
+  // A tile that is not full takes instructions of as many columns as it has (in steps of 16), and of two boxes of activation rows the
+  // first alone where that holds them: 8 192 tokens of six routes over 256 experts fill 86 % of their tiles' columns.
+  constexpr int kBoxes = NT == 64 ? 2 : 1;
+  auto cols_of = [&](int ct) { return min((2 * max(tiles[ct * 3 + 2], 1) + 15) & ~15, 2 * NT); };
   extern __shared__ uint8_t mx_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(mx_smem_raw) + 1023) & ~uintptr_t(1023));
   __nv_bfloat16* xch = reinterpret_cast<__nv_bfloat16*>(smem + kStages * S::kStageBytes);
@@ -235,15 +243,18 @@ moe_mx_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         const long long wrow = ((long long)e * row_tiles + rt) * nchunks * 128;  // first row of the item's first chunk
         const uint8_t* sa = sfa + ((size_t)e * row_tiles + rt) * nchunks * 512;
         const uint8_t* sb = sfb + (size_t)ct * nchunks * 512;
+        const int boxes = kBoxes == 2 && cols_of(ct) <= NT ? 1 : kBoxes;
         for (int sg = 0; sg < nstages; ++sg, ++ps) {
           const int s = (int)(ps % kStages);
           if (!mbar_wait(&empty[s], ((uint32_t)(ps / kStages) & 1) ^ 1, abort_flag, 21)) { ok = false; break; }
           uint8_t* st = smem + s * S::kStageBytes;
-          mbar_expect_tx(&full[s], S::kStageTxBytes);
+          mbar_expect_tx(&full[s], S::kStageTxBytes - (kBoxes - boxes) * (S::kBBytes / 2));
           tma_load_2d(st, &tmW, &full[s], 0, (int)(wrow + sg * (kChunks * 128)));  // 16 KiB of consecutive bytes
 #pragma unroll
           for (int c = 0; c < kChunks; ++c)
-            tma_load_2d(st + S::kABytes + c * (2 * NT * 128), &tmX, &full[s], (sg * kChunks + c) * 128, 2 * tok0);
+            for (int x = 0; x < boxes; ++x)
+              tma_load_2d(st + S::kABytes + c * (2 * NT * 128) + x * (2 * NT * 128 / kBoxes), &tmX, &full[s],
+                          (sg * kChunks + c) * 128, 2 * tok0 + x * (2 * NT / kBoxes));
           bulk_load(st + S::kABytes + S::kBBytes, sa + (size_t)sg * S::kSfBytes, S::kSfBytes, &full[s]);
           bulk_load(st + S::kABytes + S::kBBytes + S::kSfBytes, sb + (size_t)sg * S::kSfBytes, S::kSfBytes, &full[s]);
         }
@@ -260,6 +271,7 @@ moe_mx_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         if (!mbar_wait(&tempty[acc], ((uint32_t)(it / kAccSets) & 1) ^ 1, abort_flag, 22)) break;
         tc_fence_after();
         const uint32_t d = tmem_base + acc * S::kAccStride;
+        const uint32_t idesc = umma_idesc_mx(128, cols_of(wk / row_tiles), 5, 0);  // e2m1 x e4m3, ue8m0 scales
         bool first = true;
         for (int sg = 0; sg < nstages; ++sg) {
           const long long ps = ps0 + sg;
@@ -279,7 +291,7 @@ moe_mx_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 #pragma unroll
             for (int k = 0; k < 4; ++k)  // descriptors advance in 16-byte units: 32 bytes per K step
               umma_mx(d, a0 + (uint64_t)(c * (128 * 128 / 16) + k * 2), b0 + (uint64_t)(c * (2 * NT * 128 / 16) + k * 2),
-                      kIdesc, k, sft + c * 8, sft + c * 8 + 4, !(first && c == 0 && k == 0));
+                      idesc, k, sft + c * 8, sft + c * 8 + 4, !(first && c == 0 && k == 0));
           }
           first = false;
           umma_commit(&empty[s]);
@@ -313,28 +325,34 @@ moe_mx_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         const int orow = rt * 128 + r;
         __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out);
 #pragma unroll 1
-        for (int r0 = 0; r0 < NT; r0 += 8) {
-          if (r0 >= ntok) break;
-          float y[8];
-          load8(d0, r0, y);
+        for (int r1 = 0; r1 < ntok; r1 += 32) {
+          // lane l holds route l of the next 32 and its weight
+          const int pos = tok0 + r1 + lane;
+          int route_l = -1;
+          float w_l = 0.f;
+          if (r1 + lane < ntok) {
+            route_l = sorted_route[pos], w_l = sorted_w[pos];
+            if (route_l < 0 || route_l >= routes) dsv4_set_error(DSV4_ERR_BAD_INDEX, 35, pos), route_l = -1;
+          }
+#pragma unroll 1
+          for (int r0 = r1; r0 < min(r1 + 32, ntok); r0 += 8) {
+            float y[8];
+            load8(d0, r0, y);
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            if (r0 + c < ntok) {
-              const int pos = tok0 + r0 + c;
-              const int route = sorted_route[pos];
-              if (route >= 0 && route < routes)
-                o[(size_t)route * ld_out + orow] = __hmul(f2bf(y[c]), f2bf(sorted_w[pos]));
-              else
-                dsv4_set_error(DSV4_ERR_BAD_INDEX, 35, pos);
+            for (int c = 0; c < 8; ++c) {
+              const int route = __shfl_sync(0xffffffffu, route_l, r0 - r1 + c);
+              const float w = __shfl_sync(0xffffffffu, w_l, r0 - r1 + c);
+              if (route >= 0) o[(size_t)route * ld_out + orow] = __hmul(f2bf(y[c]), f2bf(w));
             }
           }
         }
       } else {
         // SwiGLU and the hi / lo split, kPass routes at a time.  Step 1, all four warps: the bf16-rounded sums of
         // the pass go to shared memory, xs[row][route] (gate rows 0..63, up rows 64..127; a row's entries are rotated
-        // by the row number, which spreads the lanes' column-wise stores over the banks).  Step 2, warps 0 and 1 of the
-        // group: thread (block b, route) reads its 32 gate and 32 up values, applies the clamped SwiGLU, takes the
-        // block's largest magnitude in registers and stores 32 hi and 32 lo bytes as two 16-byte pieces each.
+        // by the row number, which spreads the lanes' column-wise stores over the banks).  Step 2: a thread reads the 16 gate
+        // and 16 up values of half a block of one route and applies the clamped SwiGLU; the block's largest magnitude is that of
+        // two lanes; it stores 16 hi and 16 lo bytes.  (Two of the four warps with a whole block per thread: GEMM1 of 8 192
+        // tokens took 2 080 us, 1 930 us so.)
         constexpr int kPass = S::kPass;
         bool dead = false;
 #pragma unroll 1
@@ -353,15 +371,17 @@ moe_mx_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           __syncwarp();
           if (lane == 0) mbar_arrive(&xfull[0]);
           if (!mbar_wait(&xfull[0], (uint32_t)xph & 1, abort_flag, 25)) { dead = true; break; }
-          const int n = p0 + lane;  // route of the tile
-          if (q < 2 && lane < kPass && n < ntok) {
-            const int b = q;
-            float a[32], amax = 0.f;
+          // thread: K block, half of it, route
+          constexpr int kHalf = kPass / 2;
+          const int b = q >> 1, half = lane / kHalf, r0 = (q & 1) * kHalf + lane % kHalf, n = p0 + r0;
+          if (half < 2) {          // lanes of a block's two halves come together (narrow passes leave lanes idle)
+            const bool live = n < ntok;
+            float a[16], amax = 0.f;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int rg = b * 32 + i, ru = 64 + rg;
-              float gv = bf2f(xch[rg * kPass + ((lane + rg) & (kPass - 1))]);
-              float uv = bf2f(xch[ru * kPass + ((lane + ru) & (kPass - 1))]);
+            for (int i = 0; i < 16; ++i) {
+              const int rg = b * 32 + half * 16 + i, ru = 64 + rg;
+              float gv = bf2f(xch[rg * kPass + ((r0 + rg) & (kPass - 1))]);
+              float uv = bf2f(xch[ru * kPass + ((r0 + ru) & (kPass - 1))]);
               if (limit > 0.f) {
                 gv = fminf(gv, limit);
                 uv = fminf(fmaxf(uv, -limit), limit);
@@ -369,26 +389,29 @@ moe_mx_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
               a[i] = bf2f(f2bf(gv / (1.f + expf(-gv)) * uv));
               amax = fmaxf(amax, fabsf(a[i]));
             }
-            int eh, el;
-            mx_block_exps(amax, eh, el);
-            uint32_t wh[8] = {0, 0, 0, 0, 0, 0, 0, 0}, wl[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            amax = fmaxf(amax, __shfl_xor_sync(kPass == 32 ? 0xffffffffu : (1u << (kPass & 31)) - 1u, amax, kHalf));
+            if (live) {
+              int eh, el;
+              mx_block_exps(amax, eh, el);
+              uint32_t wh[4] = {0, 0, 0, 0}, wl[4] = {0, 0, 0, 0};
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              uint32_t hb, lb;
-              mx_split(a[i], eh, el, hb, lb);
-              wh[i >> 2] |= hb << (8 * (i & 3));
-              wl[i >> 2] |= lb << (8 * (i & 3));
+              for (int i = 0; i < 16; i += 2) {
+                uint32_t hb, lb;
+                mx_split2(a[i], a[i + 1], eh, el, hb, lb);
+                wh[i >> 2] |= hb << (8 * (i & 3));
+                wl[i >> 2] |= lb << (8 * (i & 3));
+              }
+              const int col0 = rt * 64 + b * 32;  // first intermediate index of the block
+              uint8_t* act = reinterpret_cast<uint8_t*>(out) + col0 + half * 16;
+              *reinterpret_cast<uint4*>(act + (size_t)(2 * (tok0 + n)) * ld_out) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+              *reinterpret_cast<uint4*>(act + (size_t)(2 * (tok0 + n) + 1) * ld_out) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+              if (half == 0) {
+                uint8_t* sblk = sf_out + ((size_t)ct * (rows_per_expert / 128) + col0 / 128) * 512;
+                const int kb = (col0 >> 5) & 3;
+                sblk[sf_offset(2 * n, kb)] = (uint8_t)eh;
+                sblk[sf_offset(2 * n + 1, kb)] = (uint8_t)el;
+              }
             }
-            const int col0 = rt * 64 + b * 32;  // first intermediate index of the block
-            uint8_t* act = reinterpret_cast<uint8_t*>(out);
-            uint4* dh = reinterpret_cast<uint4*>(act + (size_t)(2 * (tok0 + n)) * ld_out + col0);
-            uint4* dl = reinterpret_cast<uint4*>(act + (size_t)(2 * (tok0 + n) + 1) * ld_out + col0);
-            dh[0] = make_uint4(wh[0], wh[1], wh[2], wh[3]), dh[1] = make_uint4(wh[4], wh[5], wh[6], wh[7]);
-            dl[0] = make_uint4(wl[0], wl[1], wl[2], wl[3]), dl[1] = make_uint4(wl[4], wl[5], wl[6], wl[7]);
-            uint8_t* sblk = sf_out + ((size_t)ct * (rows_per_expert / 128) + col0 / 128) * 512;
-            const int kb = (col0 >> 5) & 3;
-            sblk[sf_offset(2 * n, kb)] = (uint8_t)eh;
-            sblk[sf_offset(2 * n + 1, kb)] = (uint8_t)el;
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(&xfull[1]);
@@ -428,7 +451,7 @@ int launch_mx_gemm(const void* w, const uint8_t* sfa, const void* xq, const uint
   // tile-major weights: every 128 rows x 64 bytes are one K chunk of one work item, chunks of an item follow each other
   const uint64_t wrows = (uint64_t)e_local * (rows_per_expert / (MODE == 1 ? 64 : 128)) * (K / 128) * 128;
   if (dsv4_make_tmap_2d(&tmW, w, 3, 128, wrows, 64, 128, S::kChunks * 128, 3)) return 241;
-  if (dsv4_make_tmap_2d(&tmX, xq, 0, (uint64_t)K, (uint64_t)2 * x_rows, (uint64_t)K, 128, 2 * NT, 3)) return 242;
+  if (dsv4_make_tmap_2d(&tmX, xq, 0, (uint64_t)K, (uint64_t)2 * x_rows, (uint64_t)K, 128, NT == 64 ? NT : 2 * NT, 3)) return 242;
   auto kern = moe_mx_gemm_kernel<MODE, NT>;
   static bool set = false;
   if (!set) {
@@ -449,12 +472,12 @@ int launch_mx_gemm(const void* w, const uint8_t* sfa, const void* xq, const uint
 DSV4_API int dsv4_moe_mx_permute(const void* x, void* xq, void* sf, const int* plan, int routes, int max_tiles, int topk,
                                  int h, int nt, cudaStream_t st) {
   if (routes <= 0) return 0;
-  if (h % 128 || (nt != 8 && nt != 16 && nt != 32 && nt != 64)) return 240;
+  if (h % 128 || (nt != 8 && nt != 16 && nt != 32 && nt != 64) || topk < 1 || topk > kMaxTopk || routes % topk) return 240;
   const MxPlanHeader* hdr = reinterpret_cast<const MxPlanHeader*>(plan);
   const int* tiles = plan + 4;
-  const int* sorted_route = tiles + 3 * max_tiles;
-  dsv4_launch(moe_mx_permute_kernel, routes, 128, 0, st, (const __nv_bfloat16*)x, (uint8_t*)xq, (uint8_t*)sf, hdr, tiles,
-              sorted_route, topk, h, routes, max_tiles, nt);
+  const int* route_pos = tiles + 3 * max_tiles + routes;
+  dsv4_launch(moe_mx_permute_kernel, routes / topk, 128, 0, st, (const __nv_bfloat16*)x, (uint8_t*)xq, (uint8_t*)sf, hdr, tiles,
+              route_pos, topk, h, routes, max_tiles, nt);
   return (int)cudaGetLastError();
 }
 
