@@ -16,7 +16,8 @@ def test_plan(routes, e, base, nt):
     w = torch.rand(routes, generator=g)
     tiles = min(e, routes) + routes // nt + 1
     plan = torch.full((4 + 3 * tiles + 3 * routes,), -9, dtype=torch.int32, device=DEV)
-    nv.call("moe_plan", nv.ptr(idx.to(DEV)), nv.ptr(w.to(DEV)), nv.I(routes), nv.I(e), nv.I(base), nv.I(nt), nv.ptr(plan), nv.I(tiles))
+    held = idx.to(DEV), w.to(DEV)
+    nv.call("moe_plan", nv.ptr(held[0]), nv.ptr(held[1]), nv.I(routes), nv.I(e), nv.I(base), nv.I(nt), nv.ptr(plan), nv.I(tiles))
     plan = plan.cpu()
     local = (idx >= base) & (idx < base + e)
     n_tiles, n = plan[:2].tolist()
