@@ -16,9 +16,10 @@
 // A key tile is 128 KiB, so one is resident: its blocks are refilled one after the other as the product with P frees them, under the
 // rest of that product, and the next token's first tile loads under this one's epilogue.  CTAs stay and walk (token, split) items.
 //
-// What bounds it: the chain gather -> S -> softmax -> PV of a tile; shared memory feeds an instruction of 64 columns at two thirds
-// of the tensor core's rate.  8 prompts of 1 024 tokens (4:1 entries): 940 us, against 2 340 us on the warp-level kernel
-// (attention.cu), which spends four barriers on every 32 keys; 128 decoded tokens at 2 000: 48 and 87 us; one token: 26 and 51 us.
+// What bounds it: the chain gather -> S -> softmax -> PV of a tile, and a token's epilogue, whose stores share the load/store path with
+// the next gather; shared memory feeds an instruction of 64 columns at two thirds of the tensor core's rate.  8 prompts of 1 024
+// tokens (4:1 entries): 800 us, against 2 340 us on the warp-level kernel (attention.cu), which spends four barriers on every 32 keys;
+// 128 decoded tokens at 2 000: 40 and 87 us; one token: 16 and 51 us.
 // The warp-level kernel stays for 8 to 32 heads, where columns would be padding.
 //
 // Splits leave unnormalised sums (fp32) with (reference, sum) per head; a second kernel merges them, four heads to a CTA.
@@ -41,16 +42,16 @@ struct TcSmem {
   uint8_t p[KT * 128];          // [key][64 heads] weights
   uint8_t ones[1024];           // an 8-row group of ones; every group of the operand is this one
   float wmax[8][32], ref[8][32], mul[8][32];
-  int valid[KT];
+  const __nv_bfloat16* rows[2][KT];     // cache rows of a tile's keys, null if masked
   uint64_t full[4], empty[4], s_full, p_full, o_full;
   uint32_t tmem;
   int abort_flag;
 };
 constexpr int kSmemBytes = (int)sizeof(TcSmem) + 1024;
 
-__device__ __forceinline__ void cp16(void* smem, const void* g, bool valid) {
+__device__ __forceinline__ void cp16(uint32_t smem, const void* g, bool valid) {
   const int sz = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem)), "l"(g), "r"(sz) : "memory");
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem), "l"(g), "r"(sz) : "memory");
 }
 __device__ __forceinline__ float redux_max(float v) {
   float r;
@@ -115,120 +116,124 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_mma_kernel(const Attn
   pdl_launch_dependents();
 
   if (warp >= 9) {
-    const int db = warp - 9;                                   // dims [128 db, +128)
+    const int db = warp - 9, mine = threadIdx.x - 9 * 32;      // dims [128 db, +128); the key of a tile that this thread looks up
     const int rpp = a.ratio > 0 ? max(a.ps / a.ratio, 1) : 1;
     const int side = lane >> 4, ch = lane & 15;                // two rows of 16 pieces at a time
-    uint8_t* kb = sm.k + 2 * db * kSub + (ch >> 3) * kSub;
-    uint8_t* qb = sm.q + 2 * db * kQSub + (ch >> 3) * kQSub;
-    constexpr int kSwa = 1 << 30;
-    int fill = 0;
+    const uint32_t kb = smem_u32(sm.k + (2 * db + (ch >> 3)) * kSub) + side * 128;
+    const uint32_t qb = smem_u32(sm.q + (2 * db + (ch >> 3)) * kQSub) + side * 128;
+    uint32_t turn[4];                                          // place of the piece in rows 2 i + side, i % 4
+#pragma unroll
+    for (int i = 0; i < 4; ++i) turn[i] = ((ch ^ (2 * i + side)) & 7) << 4;
+    // Cache row of key base + mine of an item, null if it is masked.  The chain of two or three dependent loads (behind an item's own)
+    // runs one tile ahead.
+    auto look_up = [&](const Item& x, int base) -> const __nv_bfloat16* {
+      const int key = base + mine;
+      if (key >= x.hi) return nullptr;
+      const int* pt = a.page_table + (size_t)x.slot * a.ld_pt;
+      if (key >= x.nc) {
+        const int loc = pt[x.pos - x.ns + 1 + (key - x.nc)];
+        const int sl = loc >= 0 ? a.swa_map[loc / a.ps] : -1;
+        return sl >= 0 ? a.swa + ((size_t)sl * a.ps + loc % a.ps) * D : nullptr;
+      }
+      const int j = a.mode == 1 ? a.topk_idx[(size_t)x.t * a.topk_width + key] : key;
+      const int loc = j >= 0 ? pt[j * a.ratio + a.ratio - 1] : -1;
+      return loc >= 0 ? a.comp + ((size_t)(loc / a.ps) * rpp + (loc % a.ps) / a.ratio) * D : nullptr;
+    };
+    int fill = 0, id = blockIdx.x;
+    Item x;
+    auto next_item = [&]() {                                   // the first one with keys from id on
+      for (; id < items; id += gridDim.x) {
+        x = item_of(a, id);
+        if (x.lo < x.hi) return;
+      }
+    };
+    next_item();
+    int base = id < items ? x.lo : 0;
+    const __nv_bfloat16* row = id < items ? look_up(x, base) : nullptr;
+    while (id < items) {
+      // after a wait that ran out the warps still meet here, and copy nothing
+      const __nv_bfloat16** rows = sm.rows[fill & 1];
+      rows[mine] = row;
+      asm volatile("bar.sync 3, 128;" ::: "memory");
+      if (mbar_wait<20>(&sm.empty[db], (fill & 1) ^ 1, abort_flag, 51)) {
+        if (base == x.lo) {
+          const __nv_bfloat16* q = a.q + ((size_t)x.t * HL + side) * D + db * 128 + ch * 8;
+#pragma unroll 1
+          for (int i0 = 0; i0 < 32; i0 += 4)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) cp16(qb + (i0 + i) * 256 + turn[i], q + (size_t)(i0 + i) * (2 * D), true);
+        }
+#pragma unroll 1
+        for (int i0 = 0; i0 < 64; i0 += 8) {
+          const __nv_bfloat16* r[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) r[i] = rows[2 * (i0 + i) + side];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            cp16(kb + (i0 + i) * 256 + turn[i & 3], (r[i] ? r[i] : a.swa) + db * 128 + ch * 8, r[i] != nullptr);
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      base += KT;
+      if (base >= x.hi) {
+        id += gridDim.x;
+        next_item();
+        base = x.lo;
+      }
+      if (id < items) row = look_up(x, base);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.full[db]);
+      ++fill;
+    }
+  } else if (warp == 8) {
+    // all lanes walk these loops (elect_one)
+    constexpr uint32_t kIdS = umma_idesc(128, HL, 1, 1);
+    constexpr uint32_t kIdO = kIdS | (1u << 15) | (1u << 16);       // both operands M- / N-major
+    constexpr uint32_t kIdL = kIdS | (1u << 16);
+    const uint64_t ones = desc_ones(sm.ones), k_rows = umma_desc_k128(sm.k, 0), q_rows = umma_desc_k128(sm.q, 0);
+    const uint64_t k_cols = desc_mn(sm.k), p_cols = desc_mn(sm.p);
+    const bool lead = elect_one();
+    int n = 0;
     bool ok = true;
     for (int id = blockIdx.x; id < items && ok; id += gridDim.x) {
       const Item x = item_of(a, id);
-      const int* pt = a.page_table + (size_t)x.slot * a.ld_pt;
-      // cache rows of the lane's four keys of the tile at `base` (-1: masked); the chain of two or three dependent loads runs one
-      // tile ahead
-      int row[4];
-      auto resolve = [&](int base) {
-        int at[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int key = base + 32 * u + lane;
-          at[u] = -1;
-          if (key < x.hi) {
-            if (key >= x.nc)
-              at[u] = x.pos - x.ns + 1 + (key - x.nc);
-            else {
-              const int j = a.mode == 1 ? a.topk_idx[(size_t)x.t * a.topk_width + key] : key;
-              if (j >= 0) at[u] = j * a.ratio + a.ratio - 1;
-            }
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) at[u] = at[u] >= 0 ? pt[at[u]] : -1;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int key = base + 32 * u + lane;
-          row[u] = -1;
-          if (at[u] >= 0) {
-            if (key < x.nc) {
-              row[u] = (at[u] / a.ps) * rpp + (at[u] % a.ps) / a.ratio;
-            } else {
-              const int sl = a.swa_map[at[u] / a.ps];
-              if (sl >= 0) row[u] = (sl * a.ps + at[u] % a.ps) | kSwa;
-            }
-          }
-        }
-      };
-      if (x.lo < x.hi) resolve(x.lo);
-      for (int base = x.lo; base < x.hi; base += KT, ++fill) {
-        ok = mbar_wait<20>(&sm.empty[db], (fill & 1) ^ 1, abort_flag, 51);
-        if (!ok) break;
-        if (base == x.lo) {
-          const __nv_bfloat16* q = a.q + (size_t)x.t * HL * D + db * 128 + ch * 8;
-#pragma unroll 8
-          for (int i = 0; i < 32; ++i) {
-            const int h = 2 * i + side;
-            cp16(qb + h * 128 + (((ch ^ h) & 7) << 4), q + (size_t)h * D, true);
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          const int e = __shfl_sync(0xffffffffu, row[i >> 4], (2 * i + side) & 31);
-          const int r = 2 * i + side;
-          const __nv_bfloat16* src = (e >= 0 && !(e & kSwa) ? a.comp + (size_t)e * D : a.swa + (size_t)(e >= 0 ? e & (kSwa - 1) : 0) * D);
-          cp16(kb + r * 128 + (((ch ^ r) & 7) << 4), src + db * 128 + ch * 8, e >= 0);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (db == 0) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) sm.valid[32 * u + lane] = row[u] >= 0;
-        }
-        if (base + KT < x.hi) resolve(base + KT);
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.full[db]);
-      }
-    }
-  } else if (warp == 8) {
-    if (lane == 0) {
-      constexpr uint32_t kIdS = umma_idesc(128, HL, 1, 1);
-      constexpr uint32_t kIdO = kIdS | (1u << 15) | (1u << 16);       // both operands M- / N-major
-      constexpr uint32_t kIdL = kIdS | (1u << 16);
-      const uint64_t ones = desc_ones(sm.ones);
-      int n = 0;
-      bool ok = true;
-      for (int id = blockIdx.x; id < items && ok; id += gridDim.x) {
-        const Item x = item_of(a, id);
-        for (int base = x.lo; base < x.hi && ok; base += KT, ++n) {
-          for (int db = 0; db < 4 && ok; ++db) {
-            ok = mbar_wait(&sm.full[db], n & 1, abort_flag, 52);
-            if (!ok) break;
-            tc_fence_after();
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-              umma_f16(tmem + kColS, umma_desc_k128(sm.k + (2 * db + (k >> 2)) * kSub, (k & 3) * 32),
-                       umma_desc_k128(sm.q + (2 * db + (k >> 2)) * kQSub, (k & 3) * 32), kIdS, db > 0 || k > 0);
-          }
-          if (!ok) break;
-          umma_commit(&sm.s_full);
-          ok = mbar_wait(&sm.p_full, n & 1, abort_flag, 53);
+      for (int base = x.lo; base < x.hi && ok; base += KT, ++n) {
+#pragma unroll 1
+        for (int db = 0; db < 4 && ok; ++db) {
+          ok = mbar_wait(&sm.full[db], n & 1, abort_flag, 52);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t more = base > x.lo;
-#pragma unroll
-          for (int mb = 0; mb < 4; ++mb) {
+          const uint64_t ka = k_rows + (uint64_t)(db * (2 * kSub / 16)), qa = q_rows + (uint64_t)(db * (2 * kQSub / 16));
+          if (lead) {
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-              umma_f16(tmem + kColO + mb * HL, desc_mn(sm.k + 2 * mb * kSub + k * 2048), desc_mn(sm.p + k * 2048), kIdO, more || k > 0);
+              umma_f16(tmem + kColS, ka + (k >> 2) * (kSub / 16) + (k & 3) * 2, qa + (k >> 2) * (kQSub / 16) + (k & 3) * 2, kIdS,
+                       db > 0 || k > 0);
+          }
+        }
+        if (!ok) break;
+        if (lead) umma_commit(&sm.s_full);
+        ok = mbar_wait(&sm.p_full, n & 1, abort_flag, 53);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t more = base > x.lo;
+#pragma unroll 1
+        for (int mb = 0; mb < 4; ++mb) {
+          const uint64_t va = k_cols + (uint64_t)(mb * (2 * kSub / 16));
+          if (lead) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) umma_f16(tmem + kColO + mb * HL, va + k * 128, p_cols + k * 128, kIdO, more || k > 0);
             umma_commit(&sm.empty[mb]);
           }
-#pragma unroll
-          for (int k = 0; k < 8; ++k) umma_f16(tmem + kColL, ones, desc_mn(sm.p + k * 2048), kIdL, more || k > 0);
         }
-        if (ok && x.lo < x.hi) umma_commit(&sm.o_full);
+        if (lead) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) umma_f16(tmem + kColL, ones, p_cols + k * 128, kIdL, more || k > 0);
+        }
       }
+      if (lead && ok && x.lo < x.hi) umma_commit(&sm.o_full);
     }
   } else {
     const int hf = warp >> 2, q = warp & 3, key = q * 32 + lane;
@@ -260,7 +265,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_mma_kernel(const Attn
         float s[32];
         tmem_ld_32x32(lanes + kColS, r);
         tmem_ld_wait();
-        const bool valid = sm.valid[key] != 0;
+        const bool valid = sm.rows[n & 1][key] != nullptr;
 #pragma unroll
         for (int j = 0; j < 32; ++j) s[j] = valid ? __uint_as_float(r[j]) * scale2 : -INFINITY;
         float mx = -INFINITY;
