@@ -14,7 +14,7 @@
 //   warp 1      tcgen05.mma issuer:  S_t = Q_t K^T,  O_t += P_t V  (P_t is read from tensor memory)
 //   warps 2-5   softmax of tile 0, warps 6-9 of tile 1: one thread per row; P_t overwrites S_t in place as bf16
 // The softmax warps' instructions bound it: multiplications and additions are issued two at a time (8 192 tokens of 16 heads of 128
-// with capped scores 384 us, 446 us one at a time).
+// with capped scores 384 us, 446 us one at a time; 356 us since the issuer's warp walks its loops as a whole).
 // Tensor memory: S0 | S1 | O0 | O1, 128 columns each.  O stays there; it is rescaled only when a row's maximum has grown by
 // more than 2^8 since the last time (the sums stay far from overflow, the quotient does not depend on it).
 #include "mma16.cuh"
@@ -128,56 +128,57 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t kIdS = umma_idesc(128, kQT, 1, 1);
-      const uint32_t id_o = umma_idesc(128, vp, 1, 1);
-      auto scores = [&](int t, int i) {
-        const uint8_t* kt = ks + (i & 1) * C::kK;
+    const bool lead = elect_one();      // all lanes walk these loops
+    constexpr uint32_t kIdS = umma_idesc(128, kQT, 1, 1);
+    const uint32_t id_o = umma_idesc(128, vp, 1, 1);
+    auto scores = [&](int t, int i) {
+      const uint64_t qd = umma_desc_k128(qs + t * NB * kBlk, 0), kd = umma_desc_k128(ks + (i & 1) * C::kK, 0);
+      if (lead) {
 #pragma unroll
         for (int k = 0; k < NB * 4; ++k)
-          umma_f16(tmem + t * 128, umma_desc_k128(qs + (t * NB + k / 4) * kBlk, (k & 3) * 32),
-                   umma_desc_k128(kt + k / 4 * kBlk, (k & 3) * 32), kIdS, k > 0);
-      };
-      auto values = [&](int t, int i) {
-        const uint8_t* vt = vs + (i & 1) * C::kV;
+          umma_f16(tmem + t * 128, qd + k / 4 * (kBlk / 16) + (k & 3) * 2, kd + k / 4 * (kBlk / 16) + (k & 3) * 2, kIdS, k > 0);
+      }
+    };
+    auto values = [&](int t, int i) {
+      const uint64_t vd = umma_desc_k128(vs + (i & 1) * C::kV, 0);
+      if (lead) {
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          umma_f16_ta(tmem + kColO + t * 128, tmem + t * 128 + k * 8,
-                      umma_desc_k128(vt + k / 4 * kBlk, (k & 3) * 32), id_o, i > 0 || k > 0);
-      };
-      bool ok = mbar_wait(&b->q_full, 0, abort_flag, 83) && mbar_wait(&b->k_full[0], 0, abort_flag, 84);
-      tc_fence_after();
-      if (ok) {
-        for (int t = 0; t < 2; ++t) {
-          scores(t, 0);
-          umma_commit(&b->s_full[t]);
-        }
-        umma_commit(&b->k_empty[0]);
+          umma_f16_ta(tmem + kColO + t * 128, tmem + t * 128 + k * 8, vd + k / 4 * (kBlk / 16) + (k & 3) * 2, id_o, i > 0 || k > 0);
       }
-      for (int i = 0; i < n && ok; ++i) {
-        const bool more = i + 1 < n;
-        ok = mbar_wait(&b->v_full[i & 1], (i >> 1) & 1, abort_flag, 85);
-        for (int t = 0; t < 2 && ok; ++t) {
-          ok = mbar_wait(&b->p_ready[t], i & 1, abort_flag, 86);
+    };
+    bool ok = mbar_wait(&b->q_full, 0, abort_flag, 83) && mbar_wait(&b->k_full[0], 0, abort_flag, 84);
+    tc_fence_after();
+    if (ok) {
+      for (int t = 0; t < 2; ++t) {
+        scores(t, 0);
+        if (lead) umma_commit(&b->s_full[t]);
+      }
+      if (lead) umma_commit(&b->k_empty[0]);
+    }
+    for (int i = 0; i < n && ok; ++i) {
+      const bool more = i + 1 < n;
+      ok = mbar_wait(&b->v_full[i & 1], (i >> 1) & 1, abort_flag, 85);
+      for (int t = 0; t < 2 && ok; ++t) {
+        ok = mbar_wait(&b->p_ready[t], i & 1, abort_flag, 86);
+        if (!ok) break;
+        tc_fence_after();
+        values(t, i);
+        if (more) {
+          // S_t may only be written now: P_t, which sits on it, has been consumed by the product before (MMAs of one
+          // thread run in order)
+          if (t == 0) ok = mbar_wait(&b->k_full[(i + 1) & 1], ((i + 1) >> 1) & 1, abort_flag, 87);
           if (!ok) break;
           tc_fence_after();
-          values(t, i);
-          if (more) {
-            // S_t may only be written now: P_t, which sits on it, has been consumed by the product before (MMAs of one
-            // thread run in order)
-            if (t == 0) ok = mbar_wait(&b->k_full[(i + 1) & 1], ((i + 1) >> 1) & 1, abort_flag, 87);
-            if (!ok) break;
-            tc_fence_after();
-            scores(t, i + 1);
-            umma_commit(&b->s_full[t]);
-          } else {
-            umma_commit(&b->o_full[t]);
-          }
+          scores(t, i + 1);
+          if (lead) umma_commit(&b->s_full[t]);
+        } else {
+          if (lead) umma_commit(&b->o_full[t]);
         }
-        if (ok) {
-          umma_commit(&b->v_empty[i & 1]);
-          if (more) umma_commit(&b->k_empty[(i + 1) & 1]);
-        }
+      }
+      if (ok) {
+        if (lead) umma_commit(&b->v_empty[i & 1]);
+        if (more && lead) umma_commit(&b->k_empty[(i + 1) & 1]);
       }
     }
   } else {

@@ -76,26 +76,27 @@ __global__ void __launch_bounds__(192, 1) gemm_prefill_kernel(const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t kIdesc = umma_idesc(128, kPN, 1, 1);
-      int i = 0, it = 0;
-      bool ok = true;
-      for (int id = blockIdx.x; id < total && ok; id += gridDim.x, ++it) {
-        const int acc = it & 1;
-        if (it >= 2 && !mbar_wait(&tempty[acc], ((it >> 1) & 1) ^ 1, abort_flag, 92)) break;
+    const bool lead = elect_one();      // all lanes walk these loops
+    constexpr uint32_t kIdesc = umma_idesc(128, kPN, 1, 1);
+    int i = 0, it = 0;
+    bool ok = true;
+    for (int id = blockIdx.x; id < total && ok; id += gridDim.x, ++it) {
+      const int acc = it & 1;
+      if (it >= 2 && !mbar_wait(&tempty[acc], ((it >> 1) & 1) ^ 1, abort_flag, 92)) break;
+      tc_fence_after();
+      for (int k = 0; k < nkt; ++k, ++i) {
+        const int s = i % kPStages;
+        if (!mbar_wait(&full[s], (i / kPStages) & 1, abort_flag, 93)) { ok = false; break; }
         tc_fence_after();
-        for (int k = 0; k < nkt; ++k, ++i) {
-          const int s = i % kPStages;
-          if (!mbar_wait(&full[s], (i / kPStages) & 1, abort_flag, 93)) { ok = false; break; }
-          tc_fence_after();
-          const uint8_t* st = smem + s * kPStage;
+        const uint8_t* st = smem + s * kPStage;
+        const uint64_t da = umma_desc_k128(st, 0), db = umma_desc_k128(st + kPA, 0);
+        if (lead) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            umma_f16(tmem + acc * kPN, umma_desc_k128(st, j * 32), umma_desc_k128(st + kPA, j * 32), kIdesc, k > 0 || j > 0);
+          for (int j = 0; j < 4; ++j) umma_f16(tmem + acc * kPN, da + 2 * j, db + 2 * j, kIdesc, k > 0 || j > 0);
           umma_commit(&empty[s]);
         }
-        if (ok) umma_commit(&tfull[acc]);
       }
+      if (ok && lead) umma_commit(&tfull[acc]);
     }
   } else {
     const int q = warp & 3;

@@ -81,30 +81,32 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_prefill_fp8_kernel(const __g
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t kIdesc = umma_idesc_mx(kM, kN, 0, 0);
-      int i = 0, it = 0;
-      bool ok = true;
-      for (int id = blockIdx.x; id < total && ok; id += gridDim.x, ++it) {
-        const int acc = it & 1;
-        if (it >= 2 && !mbar_wait(&tempty[acc], ((it >> 1) & 1) ^ 1, abort_flag, 62)) break;
+    // all lanes walk these loops: three copies of scales and four MMAs per stage, issued by a branch of one lane, took 815 us in the four
+    // projections of an attention block, 730 us so
+    const bool lead = elect_one();
+    constexpr uint32_t kIdesc = umma_idesc_mx(kM, kN, 0, 0);
+    int i = 0, it = 0;
+    bool ok = true;
+    for (int id = blockIdx.x; id < total && ok; id += gridDim.x, ++it) {
+      const int acc = it & 1;
+      if (it >= 2 && !mbar_wait(&tempty[acc], ((it >> 1) & 1) ^ 1, abort_flag, 62)) break;
+      tc_fence_after();
+      for (int k = 0; k < nkt; ++k, ++i) {
+        const int s = i % kStages;
+        if (!mbar_wait(&full[s], (i / kStages) & 1, abort_flag, 63)) { ok = false; break; }
         tc_fence_after();
-        for (int k = 0; k < nkt; ++k, ++i) {
-          const int s = i % kStages;
-          if (!mbar_wait(&full[s], (i / kStages) & 1, abort_flag, 63)) { ok = false; break; }
-          tc_fence_after();
-          const uint8_t* st = smem + s * kPad;
-          const uint32_t sft = tmem + 2 * kN + (i & 1) * 12;
+        const uint8_t* st = smem + s * kPad;
+        const uint32_t sft = tmem + 2 * kN + (i & 1) * 12;
+        const uint64_t da = umma_desc_k128(st, 0), db = umma_desc_k128(st + kA, 0);
+        if (lead) {
 #pragma unroll
           for (int c = 0; c < 3; ++c) tmem_cp_sf(sft + 4 * c, st + kOperands + c * 512);
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            umma_mx(tmem + acc * kN, umma_desc_k128(st, j * 32), umma_desc_k128(st + kA, j * 32), kIdesc, j, sft, sft + 4,
-                    k > 0 || j > 0);
+          for (int j = 0; j < 4; ++j) umma_mx(tmem + acc * kN, da + 2 * j, db + 2 * j, kIdesc, j, sft, sft + 4, k > 0 || j > 0);
           umma_commit(&empty[s]);
         }
-        if (ok) umma_commit(&tfull[acc]);
       }
+      if (ok && lead) umma_commit(&tfull[acc]);
     }
   } else if (warp >= 6) {
     // thread r: row r of the tile, columns r and 128 + r

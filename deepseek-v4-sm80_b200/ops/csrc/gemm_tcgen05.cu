@@ -209,39 +209,39 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t d = tmem_base;
-      const uint32_t sfb_t = tmem_base + BN, sfa_t = tmem_base + BN + 4;  // scale columns behind the accumulator
-      bool ok = true;
-      if (FP8 && nkt > 0) {
-        // the scale blocks of this CTA's K range are in shared memory once the epilogue warps have arrived
-        ok = mbar_wait(&tempty[0], 0, abort_flag, 2);
-        tc_fence_after();
-        if (ok) tmem_cp_sf(sfb_t, sf_all + (size_t)nkt * 512);
-      }
-      for (int i = 0; i < nkt && ok; ++i) {
-        const int s = i % S;
-        const uint32_t ph = (i / S) & 1;
-        if (!mbar_wait(&full[s], ph, abort_flag, 3)) break;
-        tc_fence_after();
-        const uint8_t* a = tiles + s * Cfg::kStageBytes;
-        const uint8_t* bt = a + Cfg::kABytes;
-        const uint32_t sfa_i = sfa_t + (uint32_t)(i & 1) * 4;
+    const bool lead = elect_one();      // all lanes walk these loops
+    const uint32_t d = tmem_base;
+    const uint32_t sfb_t = tmem_base + BN, sfa_t = tmem_base + BN + 4;  // scale columns behind the accumulator
+    bool ok = true;
+    if (FP8 && nkt > 0) {
+      // the scale blocks of this CTA's K range are in shared memory once the epilogue warps have arrived
+      ok = mbar_wait(&tempty[0], 0, abort_flag, 2);
+      tc_fence_after();
+      if (ok && lead) tmem_cp_sf(sfb_t, sf_all + (size_t)nkt * 512);
+    }
+    for (int i = 0; i < nkt && ok; ++i) {
+      const int s = i % S;
+      const uint32_t ph = (i / S) & 1;
+      if (!mbar_wait(&full[s], ph, abort_flag, 3)) break;
+      tc_fence_after();
+      const uint8_t* a = tiles + s * Cfg::kStageBytes;
+      const uint8_t* bt = a + Cfg::kABytes;
+      const uint32_t sfa_i = sfa_t + (uint32_t)(i & 1) * 4;
+      const uint64_t ad = umma_desc_k128(a, 0), bd = umma_desc_k128(bt, 0);
+      if (lead) {
         if (FP8) tmem_cp_sf(sfa_i, sf_all + (size_t)i * 512);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const uint64_t ad = umma_desc_k128(a, k * 32);
-          const uint64_t bd = umma_desc_k128(bt, k * 32);
           const uint32_t acc = (i > 0 || k > 0);
           if (FP8)
-            umma_mx(d, ad, bd, kIdesc, k, sfa_i, sfb_t, acc);
+            umma_mx(d, ad + 2 * k, bd + 2 * k, kIdesc, k, sfa_i, sfb_t, acc);
           else
-            umma_f16(d, ad, bd, kIdesc, acc);
+            umma_f16(d, ad + 2 * k, bd + 2 * k, kIdesc, acc);
         }
         umma_commit(&empty[s]);
       }
-      if (nkt > 0) umma_commit(&tfull[0]);
     }
+    if (nkt > 0 && lead) umma_commit(&tfull[0]);
   } else {
     // epilogue warps 2..5 ; TMEM lane quarter = warp % 4
     const int q = warp & 3;

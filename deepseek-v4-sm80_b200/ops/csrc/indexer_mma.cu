@@ -171,27 +171,28 @@ indexer_logits_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer
-    if (lane == 0) {
-      bool ok = mbar_wait(qfull, 0, abort_flag, 12);
-      int it = 0;
-      for (int p = 0; p < npass && ok; ++p) {
-        const uint32_t idesc = umma_idesc(KB, HEADS * p_cnt[p], 0, 0);
-        const uint8_t* qb = qtile + p_first[p] * kQTile;
-        for (int kb = split; kb < p_blocks[p]; kb += nsplit, ++it) {
-          const int s = it % NS, b = it & 1;
-          if (!mbar_wait(&tempty[b], ((it >> 1) & 1) ^ 1, abort_flag, 13)) {
-            ok = false;
-            break;
-          }
-          if (!mbar_wait(&full[s], (it / NS) & 1, abort_flag, 14)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t d = tmem_base + b * (a.tg * HEADS);
+    const bool lead = elect_one();      // all lanes walk these loops
+    bool ok = mbar_wait(qfull, 0, abort_flag, 12);
+    int it = 0;
+    for (int p = 0; p < npass && ok; ++p) {
+      const uint32_t idesc = umma_idesc(KB, HEADS * p_cnt[p], 0, 0);
+      const uint8_t* qb = qtile + p_first[p] * kQTile;
+      for (int kb = split; kb < p_blocks[p]; kb += nsplit, ++it) {
+        const int s = it % NS, b = it & 1;
+        if (!mbar_wait(&tempty[b], ((it >> 1) & 1) ^ 1, abort_flag, 13)) {
+          ok = false;
+          break;
+        }
+        if (!mbar_wait(&full[s], (it / NS) & 1, abort_flag, 14)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t d = tmem_base + b * (a.tg * HEADS);
+        const uint64_t da = umma_desc_k128(atiles + s * kATile, 0), db = umma_desc_k128(qb, 0);
+        if (lead) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_f8(d, umma_desc_k128(atiles + s * kATile, k * 32), umma_desc_k128(qb, k * 32), idesc, k > 0);
+          for (int k = 0; k < 4; ++k) umma_f8(d, da + 2 * k, db + 2 * k, idesc, k > 0);
           umma_commit(&empty[s]);
           umma_commit(&tfull[b]);
         }

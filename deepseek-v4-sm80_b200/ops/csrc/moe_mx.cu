@@ -20,7 +20,8 @@
 //
 // "swap-AB" as in moe.cu: the 128 weight rows of a work item sit on the TMEM lanes, routes are the N dimension.
 // With a handful of routes per expert an instruction does little arithmetic, so what bounds the kernel is how fast
-// instructions are issued, not the tensor pipe.  Measured on one CTA (M = 128, K = 32, this MMA kind): one thread
+// instructions are issued, not the tensor pipe.  Measured on one CTA (M = 128, K = 32, this MMA kind): one thread, in a branch of its
+// own (a warp that walks the issuer's loops as a whole takes 48 cycles or less, elect_one: 128 tokens 551 -> 494 us, 6.5 TB/s),
 // issues an MMA every 68 cycles whatever N <= 128 is, two threads together every 39 (N = 16) to 64 cycles (N = 128,
 // the pipe's own rate), a TMA or bulk copy costs its issuing thread about 70 cycles.  Inside this kernel, with one
 // CTA per SM and 256-element stages, the issuer spent 785 cycles on a stage (8 MMAs, 4 scale copies) plus 165 on the
@@ -261,26 +262,27 @@ moe_mx_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      long long ps0 = 0;  // ring index of the work item's first stage
-      int it = 0;
-      bool ok = true;
-      const uint32_t sf_base = tmem_base + S::kAccCols;
-      for (int wk = blockIdx.x; wk < total_work && ok; wk += gridDim.x, ++it, ps0 += nstages) {
-        const int acc = it % kAccSets;
-        if (!mbar_wait(&tempty[acc], ((uint32_t)(it / kAccSets) & 1) ^ 1, abort_flag, 22)) break;
+    const bool lead = elect_one();      // all lanes walk these loops
+    long long ps0 = 0;  // ring index of the work item's first stage
+    int it = 0;
+    bool ok = true;
+    const uint32_t sf_base = tmem_base + S::kAccCols;
+    for (int wk = blockIdx.x; wk < total_work && ok; wk += gridDim.x, ++it, ps0 += nstages) {
+      const int acc = it % kAccSets;
+      if (!mbar_wait(&tempty[acc], ((uint32_t)(it / kAccSets) & 1) ^ 1, abort_flag, 22)) break;
+      tc_fence_after();
+      const uint32_t d = tmem_base + acc * S::kAccStride;
+      const uint32_t idesc = umma_idesc_mx(128, cols_of(wk / row_tiles), 5, 0);  // e2m1 x e4m3, ue8m0 scales
+      bool first = true;
+      for (int sg = 0; sg < nstages; ++sg) {
+        const long long ps = ps0 + sg;
+        const int s = (int)(ps % kStages);
+        if (!mbar_wait(&full[s], (uint32_t)(ps / kStages) & 1, abort_flag, 23)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d = tmem_base + acc * S::kAccStride;
-        const uint32_t idesc = umma_idesc_mx(128, cols_of(wk / row_tiles), 5, 0);  // e2m1 x e4m3, ue8m0 scales
-        bool first = true;
-        for (int sg = 0; sg < nstages; ++sg) {
-          const long long ps = ps0 + sg;
-          const int s = (int)(ps % kStages);
-          if (!mbar_wait(&full[s], (uint32_t)(ps / kStages) & 1, abort_flag, 23)) { ok = false; break; }
-          tc_fence_after();
-          const uint8_t* st = smem + s * S::kStageBytes;
-          const uint32_t sft = sf_base + (uint32_t)(ps & 1) * (kChunks * 8);  // the scale columns alternate per stage
-          const uint64_t a0 = umma_desc_k128(st, 0), b0 = umma_desc_k128(st + S::kABytes, 0);
+        const uint8_t* st = smem + s * S::kStageBytes;
+        const uint32_t sft = sf_base + (uint32_t)(ps & 1) * (kChunks * 8);  // the scale columns alternate per stage
+        const uint64_t a0 = umma_desc_k128(st, 0), b0 = umma_desc_k128(st + S::kABytes, 0);
+        if (lead) {
 #pragma unroll
           for (int c = 0; c < kChunks; ++c) {
             tmem_cp_sf(sft + c * 8, st + S::kABytes + S::kBBytes + c * 512);
@@ -293,11 +295,11 @@ moe_mx_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
               umma_mx(d, a0 + (uint64_t)(c * (128 * 128 / 16) + k * 2), b0 + (uint64_t)(c * (2 * NT * 128 / 16) + k * 2),
                       idesc, k, sft + c * 8, sft + c * 8 + 4, !(first && c == 0 && k == 0));
           }
-          first = false;
           umma_commit(&empty[s]);
         }
-        if (ok) umma_commit(&tfull[acc]);
+        first = false;
       }
+      if (ok && lead) umma_commit(&tfull[acc]);
     }
   } else if (warp < 6) {  // epilogue: warp w reads the TMEM lanes of quarter w % 4
     const int q = warp & 3;
@@ -429,7 +431,7 @@ moe_mx_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if (*abort_flag) {
     // a wait ran out (the status word says where): before the tensor memory is freed and the CTA leaves, let the
     // MMAs already issued retire and the copies in flight land, each with a limit of its own
-    if (warp == 1 && lane == 0) {
+    if (warp == 1 && elect_one()) {
       umma_commit(drain);
       for (int i = 0; i < 20000 && !mbar_try_wait(drain, 0); ++i) __nanosleep(100);
     }
