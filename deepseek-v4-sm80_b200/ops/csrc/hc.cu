@@ -15,8 +15,11 @@ constexpr int kM = 4;  // streams
 
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + expf(-x)); }
 
+// Latency bounds it: a chain of loads, block sums and 20 dependent Sinkhorn iterations per token, hidden by the tokens that share an SM
+// (33 KB and at most 40 registers a thread: six).  What does not depend on the row (mix sums, scales) is asked for ahead of it, and comb,
+// which nothing here needs, comes last.  7 001 rows of 4 x 4 096: 97 us, 120 us with four tokens an SM and comb ahead of y.
 template <int MIX>  // 24 = layer (pre, post, comb), 4 = head (pre only)
-__global__ void __launch_bounds__(256) hc_pre_kernel(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(256, 6) hc_pre_kernel(const __nv_bfloat16* __restrict__ x,
                                                      const __nv_bfloat16* __restrict__ fn,
                                                      const float* __restrict__ mixes_in, int ld_mix, int n_part,
                                                      long long part_stride,
@@ -29,12 +32,16 @@ __global__ void __launch_bounds__(256) hc_pre_kernel(const __nv_bfloat16* __rest
   pdl_entry();
   extern __shared__ __align__(16) uint8_t hc_smem[];
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(hc_smem);  // [4*h]
-  __shared__ float red[32];
+  __shared__ float red[32], norm[32];
   __shared__ float mixes[MIX];
   __shared__ float pre_s[kM];
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int total = kM * h;
   const __nv_bfloat16* xr = x + (size_t)t * total;
+  // split-K partial products of the mix rows: warp w adds splits w, w + 8, ..., then the eight sums are added in warp order
+  // (a fixed tree, so the result does not depend on timing)
+  float part = 0.f;
+  if (mixes_in && warp < n_part && lane < MIX) part = __ldg(mixes_in + (size_t)warp * part_stride + (size_t)t * ld_mix + lane);
   float ss = 0.f;
   for (int i = tid * 8; i < total; i += 256 * 8) {
     const uint4 u = *reinterpret_cast<const uint4*>(xr + i);
@@ -52,11 +59,9 @@ __global__ void __launch_bounds__(256) hc_pre_kernel(const __nv_bfloat16* __rest
   // mix rows: taken from a tensor-core GEMM over all tokens when the caller ran one (every CTA re-reading the
   // [MIX, 4h] matrix costs more than the rest of the kernel), else warp w computes rows w, w+8, ...
   if (mixes_in) {
-    // split-K partial products: warp w adds splits w, w + 8, ..., then the eight sums are added in warp order
-    // (a fixed tree, so the result does not depend on timing)
     __shared__ float part_s[8][32];
-    float a = 0.f;
-    for (int p0 = warp; p0 < n_part; p0 += 64) {  // eight loads in flight per thread
+    float a = part;
+    for (int p0 = warp + 8; p0 < n_part; p0 += 64) {  // eight loads in flight per thread
       float v[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
@@ -94,38 +99,11 @@ __global__ void __launch_bounds__(256) hc_pre_kernel(const __nv_bfloat16* __rest
     if (lane == 0) mixes[r] = acc;
   }
   __syncthreads();
-  if (warp == 0) {
-    float tot = (lane < 8) ? red[lane] : 0.f;
-    tot = warp_sum(tot);
-    const float r = rsqrtf(tot / (float)total + norm_eps);
-    if (lane < kM) {
-      const float pre = sigmoidf_(mixes[lane] * r * scale[0] + base[lane]) + eps;
-      pre_s[lane] = pre;
-      if (MIX == 24) post[(size_t)t * kM + lane] = 2.f * sigmoidf_(mixes[kM + lane] * r * scale[1] + base[kM + lane]);
-    }
-    if (MIX == 24) {
-      // lanes 0..15 hold comb[j][i] with j = lane / 4 (row), i = lane % 4 (column)
-      const int l16 = lane & 15;
-      float v = mixes[2 * kM + l16] * r * scale[2] + base[2 * kM + l16];
-      float mx = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-      float e = expf(v - mx);
-      float rs = e + __shfl_xor_sync(0xffffffffu, e, 1);
-      rs += __shfl_xor_sync(0xffffffffu, rs, 2);
-      float c = e / fmaxf(rs, eps) + eps;
-      float cs = c + __shfl_xor_sync(0xffffffffu, c, 4);
-      cs += __shfl_xor_sync(0xffffffffu, cs, 8);
-      c = c / (cs + eps);
-      for (int it = 0; it < iters - 1; ++it) {
-        rs = c + __shfl_xor_sync(0xffffffffu, c, 1);
-        rs += __shfl_xor_sync(0xffffffffu, rs, 2);
-        c = c / (rs + eps);
-        cs = c + __shfl_xor_sync(0xffffffffu, c, 4);
-        cs += __shfl_xor_sync(0xffffffffu, cs, 8);
-        c = c / (cs + eps);
-      }
-      if (lane < 16) comb[(size_t)t * 16 + lane] = c;
-    }
+  const float r = rsqrtf(warp_sum(lane < 8 ? red[lane] : 0.f) / (float)total + norm_eps);
+  if (warp == 0 && lane < kM) {
+    const float pre = sigmoidf_(mixes[lane] * r * scale[0] + base[lane]) + eps;
+    pre_s[lane] = pre;
+    if (MIX == 24) post[(size_t)t * kM + lane] = 2.f * sigmoidf_(mixes[kM + lane] * r * scale[1] + base[kM + lane]);
   }
   __syncthreads();
   const float p0 = pre_s[0], p1 = pre_s[1], p2 = pre_s[2], p3 = pre_s[3];
@@ -159,10 +137,9 @@ __global__ void __launch_bounds__(256) hc_pre_kernel(const __nv_bfloat16* __rest
   float rn = 1.f;
   if (norm_w) {
     ys = warp_sum(ys);
+    if (lane == 0) norm[warp] = ys;
     __syncthreads();
-    if (lane == 0) red[warp] = ys;
-    __syncthreads();
-    float tot = (lane < 8) ? red[lane] : 0.f;
+    float tot = (lane < 8) ? norm[lane] : 0.f;
     tot = warp_sum(tot);
     rn = rsqrtf(tot / (float)h + rms_eps);
   }
@@ -197,9 +174,32 @@ __global__ void __launch_bounds__(256) hc_pre_kernel(const __nv_bfloat16* __rest
       }
     }
   }
+  if (MIX == 24 && warp == 7) {
+    // lanes 0..15 hold comb[j][i] with j = lane / 4 (row), i = lane % 4 (column)
+    const int l16 = lane & 15;
+    float v = mixes[2 * kM + l16] * r * scale[2] + base[2 * kM + l16];
+    float mx = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    float e = expf(v - mx);
+    float rs = e + __shfl_xor_sync(0xffffffffu, e, 1);
+    rs += __shfl_xor_sync(0xffffffffu, rs, 2);
+    float c = e / fmaxf(rs, eps) + eps;
+    float cs = c + __shfl_xor_sync(0xffffffffu, c, 4);
+    cs += __shfl_xor_sync(0xffffffffu, cs, 8);
+    c = c / (cs + eps);
+    for (int it = 0; it < iters - 1; ++it) {
+      rs = c + __shfl_xor_sync(0xffffffffu, c, 1);
+      rs += __shfl_xor_sync(0xffffffffu, rs, 2);
+      c = c / (rs + eps);
+      cs = c + __shfl_xor_sync(0xffffffffu, c, 4);
+      cs += __shfl_xor_sync(0xffffffffu, cs, 8);
+      c = c / (cs + eps);
+    }
+    if (lane < 16) comb[(size_t)t * 16 + lane] = c;
+  }
 }
 
-__global__ void __launch_bounds__(256) hc_post_kernel(const __nv_bfloat16* __restrict__ y,
+__global__ void __launch_bounds__(256, 4) hc_post_kernel(const __nv_bfloat16* __restrict__ y,
                                                       const __nv_bfloat16* __restrict__ res,
                                                       const float* __restrict__ post, const float* __restrict__ comb,
                                                       __nv_bfloat16* __restrict__ out, int h) {
@@ -268,6 +268,7 @@ DSV4_API int dsv4_hc_pre(const void* x, const void* fn, const float* mixes, int 
     static bool set = false;
     if (!set) {
       cudaFuncSetAttribute(hc_pre_kernel<24>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 4096 * 2);
+      cudaFuncSetAttribute(hc_pre_kernel<24>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
       set = true;
     }
     dsv4_launch(hc_pre_kernel<24>, t, 256, smem, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)fn, mixes, ld_mix, n_part, part_stride, scale, base,
