@@ -21,7 +21,7 @@
 // "swap-AB" as in moe.cu: the 128 weight rows of a work item sit on the TMEM lanes, routes are the N dimension.
 // With a handful of routes per expert an instruction does little arithmetic, so what bounds the kernel is how fast
 // instructions are issued, not the tensor pipe.  Measured on one CTA (M = 128, K = 32, this MMA kind): one thread, in a branch of its
-// own (a warp that walks the issuer's loops as a whole takes 48 cycles or less, elect_one: 128 tokens 551 -> 494 us, 6.5 TB/s),
+// own (a warp that walks the issuer's loops as a whole is faster, elect_one: 128 tokens 551 -> 494 us, 6.5 TB/s),
 // issues an MMA every 68 cycles whatever N <= 128 is, two threads together every 39 (N = 16) to 64 cycles (N = 128,
 // the pipe's own rate), a TMA or bulk copy costs its issuing thread about 70 cycles.  Inside this kernel, with one
 // CTA per SM and 256-element stages, the issuer spent 785 cycles on a stage (8 MMAs, 4 scale copies) plus 165 on the
