@@ -72,7 +72,7 @@ __device__ __forceinline__ int sf_offset(int n, int kb) { return (n & 31) * 16 +
 // into the scale block of the position's route tile: sf[tile][K / 128][512] at rows 2 n and 2 n + 1, n = pos - tile start.
 // A CTA per token: its row is read and split once, for all of its routes.  8 192 tokens of six routes: 133 us, 227 us with a CTA per
 // route.
-constexpr int kMaxTopk = 32;
+constexpr int kMaxTopk = 128;     // a thread per route
 __global__ void __launch_bounds__(128) moe_mx_permute_kernel(const __nv_bfloat16* __restrict__ x,
                                                              uint8_t* __restrict__ xq, uint8_t* __restrict__ sf,
                                                              const MxPlanHeader* __restrict__ hdr,
