@@ -243,8 +243,10 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_mma_kernel(const Attn
     const float sink2 = a.sink[head] * kLog2e;
     const int d0 = q * 32 + (lane & ~1);             // first of the pair of dims (within a block of 128) that this lane stores
     int n = 0, done = 0;
+    // False after a wait that ran out.  The warps of a half still meet at every tile's barrier, which a warp that left would keep the
+    // others at for good; they wait for nothing more and store nothing.
     bool ok = true;
-    for (int id = blockIdx.x; id < items && ok; id += gridDim.x) {
+    for (int id = blockIdx.x; id < items; id += gridDim.x) {
       const Item x = item_of(a, id);
       const size_t part = (size_t)id * HL;           // [t][split][head]
       if (x.lo >= x.hi) {
@@ -258,8 +260,8 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_mma_kernel(const Attn
       }
       float ref = x.split == 0 ? sink2 : -1e30f;
       for (int base = x.lo; base < x.hi; base += KT, ++n) {
-        ok = mbar_wait<16>(&sm.s_full, n & 1, abort_flag, 54) && mbar_wait(&sm.full[0], n & 1, abort_flag, 55);
-        if (!ok) break;
+        ok = ok && mbar_wait<16>(&sm.s_full, n & 1, abort_flag, 54) && mbar_wait(&sm.full[0], n & 1, abort_flag, 55);
+        ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
         uint32_t r[32];
         float s[32];
@@ -279,6 +281,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_mma_kernel(const Attn
           asm volatile("bar.sync 2, 128;" ::: "memory");
         else
           asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (!ok) continue;
         mx = fmaxf(fmaxf(sm.wmax[hf * 4][lane], sm.wmax[hf * 4 + 1][lane]), fmaxf(sm.wmax[hf * 4 + 2][lane], sm.wmax[hf * 4 + 3][lane]));
         const bool first = base == x.lo, grow = first ? mx > ref : mx > ref + 8.f;
         const float now = grow ? mx : ref;
@@ -319,10 +322,9 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_mma_kernel(const Attn
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.p_full);
       }
-      if (!ok) break;
-      ok = mbar_wait<16>(&sm.o_full, done & 1, abort_flag, 56);
+      ok = __all_sync(0xffffffffu, ok && mbar_wait<16>(&sm.o_full, done & 1, abort_flag, 56));
       ++done;
-      if (!ok) break;
+      if (!ok) continue;
       tc_fence_after();
       float l[32];
       {
