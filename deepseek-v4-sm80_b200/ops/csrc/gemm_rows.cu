@@ -81,6 +81,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemm_rows_kernel(const RowsArg
   const int nkb = a.K / 128;
   const float* sb = FP8 ? a.sb + (size_t)(min(n0, a.N - 1) >> 7) * nkb : nullptr;
   float acc[NTL][4] = {}, sum[NTL][4] = {};
+  uint32_t bits = 0;            // of all block scales read: no sign and no mantissa if each is a power of two
   for (int s0 = lo; s0 < hi; s0 += kU) {
     uint4 wc[kU][2], xv[kU][NTL];
     float f0[kU / 2][NTL], f1[kU / 2][NTL];      // scales of a block of 128 places and this lane's two rows of X
@@ -92,10 +93,13 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemm_rows_kernel(const RowsArg
       for (int j = 0; j < NTL; ++j) xv[u][j] = *reinterpret_cast<const uint4*>(x[j] + (size_t)s * 64);
       if (FP8 && (u & 1)) {
         const float sw = sb[s >> 1];
+        bits |= __float_as_uint(sw);
 #pragma unroll
         for (int j = 0; j < NTL; ++j) {
-          f0[u >> 1][j] = a.sa[(size_t)min(8 * j + 2 * t, a.M - 1) * nkb + (s >> 1)] * sw;
-          f1[u >> 1][j] = a.sa[(size_t)min(8 * j + 2 * t + 1, a.M - 1) * nkb + (s >> 1)] * sw;
+          const float r0 = a.sa[(size_t)min(8 * j + 2 * t, a.M - 1) * nkb + (s >> 1)];
+          const float r1 = a.sa[(size_t)min(8 * j + 2 * t + 1, a.M - 1) * nkb + (s >> 1)];
+          bits |= __float_as_uint(r0) | __float_as_uint(r1);
+          f0[u >> 1][j] = r0 * sw, f1[u >> 1][j] = r1 * sw;
         }
       }
     }
@@ -134,6 +138,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemm_rows_kernel(const RowsArg
       }
     }
   }
+  if (FP8 && (bits & 0x807fffffu)) dsv4_set_error(DSV4_ERR_BAD_INDEX, 41, (int)blockIdx.x);      // a scale that is not a power of two
 #pragma unroll
   for (int j = 0; j < NTL; ++j) {
     part[warp][8 * j + 2 * t][g] = acc[j][0], part[warp][8 * j + 2 * t + 1][g] = acc[j][1];
