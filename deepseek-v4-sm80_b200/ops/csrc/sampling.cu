@@ -45,11 +45,14 @@ __device__ __forceinline__ unsigned long long block_scan_u64(unsigned long long 
   return x - v + (w ? wt[w - 1] : 0ull);
 }
 
-// Any row: the key of the last kept rank byte by byte, each byte a pass over the whole row.  Rows that the histogram below cannot
-// order come here: a maximum or a temperature that is not finite, values that are not numbers, more entries in the last kept bin
-// than its list holds (equal logits above all).
+// Any row: the key of the last kept rank byte by byte, each byte a pass over the whole row.  Rows that the kernel below cannot order come
+// here: a maximum or a temperature that is not finite, values that are not numbers, more entries around the end of the kept set than its
+// list holds (equal logits above all).  What is known by then is given: ztot, and that the last kept key is one of [kmin, kmax], which
+// cnt_above entries of mass mass_above come before.  Bytes that kmin and kmax share need no pass, so equal logits need none.
 template <class V>
-__device__ __noinline__ int sample_exhaustive(V val, int v, float mx, int amax, float temp, int tk, float tp, float u) {
+__device__ __noinline__ int sample_exhaustive(V val, int v, float mx, int amax, float temp, int tk, float tp, float u,
+                                              unsigned long long ztot, int cnt_above, unsigned long long mass_above, uint32_t kmin,
+                                              uint32_t kmax) {
   __shared__ int si[32];
   __shared__ unsigned long long wt[32];
   __shared__ unsigned long long hmass[256];
@@ -58,18 +61,15 @@ __device__ __noinline__ int sample_exhaustive(V val, int v, float mx, int amax, 
   __shared__ unsigned long long sh_mass_above;
   const int tid = threadIdx.x, lane = tid & 31;
   const float inv_t = 1.f / temp;
-  // Z in fixed point of exp((x - mx)/T)  (each term <= 1)
-  unsigned long long zl = 0;
-  for (int i = tid; i < v; i += 1024) zl += fx(expf((val(i) - mx) * inv_t));
-  unsigned long long ztot;
-  block_scan_u64(zl, wt, ztot);
   const unsigned long long p_limit = tp >= 1.f ? ~0ull : (unsigned long long)((double)ztot * (double)tp);
   const int k_limit = tk > 0 ? tk : 0x7fffffff;
   // radix descent: find the key of the last kept rank
   uint32_t prefix = 0, mask = 0;
-  int cnt_above = 0;
-  unsigned long long mass_above = 0;
   for (int shift = 24; shift >= 0; shift -= 8) {
+    if (((kmin ^ kmax) >> shift) == 0) {
+      prefix = kmin & (~0u << shift), mask = ~0u << shift;
+      continue;
+    }
     for (int i = tid; i < 256; i += 1024) hcnt[i] = 0, hmass[i] = 0ull;
     __syncthreads();
     // Histogram of the candidates' next key byte.  The top bytes of nearly all logits agree, so per-element atomics
@@ -83,7 +83,7 @@ __device__ __noinline__ int sample_exhaustive(V val, int v, float mx, int amax, 
       if (i < v) {
         const float x = val(i);
         const uint32_t key = okey(x);
-        if ((key & mask) == prefix) {
+        if ((key & mask) == prefix && key >= kmin && key <= kmax) {
           act = true;
           bin = (key >> shift) & 0xff;
           m = fx(expf((x - mx) * inv_t));
@@ -128,6 +128,7 @@ __device__ __noinline__ int sample_exhaustive(V val, int v, float mx, int amax, 
     __syncthreads();
     prefix |= (uint32_t)sh_bin << shift;
     mask |= 0xffu << shift;
+    kmin = max(kmin, prefix), kmax = min(kmax, prefix | ~mask);
     cnt_above = sh_cnt_above;
     mass_above = sh_mass_above;
     __syncthreads();
@@ -195,6 +196,7 @@ struct SampleSmem {
   unsigned long long wt[32], seg[32];
   unsigned long long mass_above, last;
   int n, bin, cnt_above, found;
+  uint32_t kmin, kmax;           // of the listed entries
 };
 
 // list[0..n) in descending order, n <= kList; all 1024 threads.
@@ -220,7 +222,8 @@ __device__ __forceinline__ float key_value(uint32_t k) { return __uint_as_float(
 // What bounds it: passes over the row, which the L2 holds after the first (128 rows of 129 280 floats: 66 MB).  A warp reads one
 // 32nd of the row, 16 bytes a lane and four loads in flight.  Two to three passes do: the maximum; the sum of the masses together
 // with a histogram of (mx - x) / T, or, for a top_k of at most 256, with the list of what reaches the k-th largest of the threads'
-// own maxima (at least k entries do); then, behind a histogram, the masses that the last kept bin's order decides.
+// own maxima (at least k entries do); then, behind a histogram, the masses that the last kept bin's order decides.  Entries without a
+// mass (-inf: a grammar's mask) are never drawn and never listed, so they do not fill the list.
 // Only that bin's entries, about 200 of them for logits of a spread of 2.5, or that list are put in order.  The pass that finds the
 // sample reads the one 32nd that it falls into.  128 rows of 129 280 at top_k 50 and top_p 0.95 take 55 us; the four passes of the
 // descent, three walks over 126 consecutive ids a thread and the passes before them took 620 us.
@@ -238,7 +241,7 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
   const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const float* row = logits + (size_t)b * v;
   const int* mrow = mask_ids ? mask_ids + (size_t)b * n_mask : nullptr;
-  auto masked = [&](float x, int i) -> float {
+  auto masked = [mrow, n_mask](float x, int i) -> float {
     for (int m = 0; m < n_mask; ++m)
       if (mrow[m] == i) x = -INFINITY;
     return x;
@@ -272,7 +275,7 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
     if (tail < hi) f(masked(row[tail], tail), tail);
   };
   // argmax (lowest id wins ties) -- also the softmax max
-  if (tid == 0) sbad = 0, sm.n = 0;
+  if (tid == 0) sbad = 0, sm.n = 0, sm.kmin = ~0u, sm.kmax = 0;
   float best = -INFINITY;
   int bi = 0x7fffffff;
   bool nan = false;
@@ -312,21 +315,31 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
   }
   const float u = uniform ? uniform[b] : 0.5f;
   const float inv_t = 1.f / temp;
-  auto exhaustive = [&]() {
-    const int id = sample_exhaustive([&](int i) { return masked(row[i], i); }, v, mx, amax, temp, tk, tp, u);
+  auto mass = [&](float x) { return fx(expf((x - mx) * inv_t)); };
+  auto exhaustive = [&](u64 ztot, int cnt_above, u64 mass_above, uint32_t kmin, uint32_t kmax) {
+    const int id = sample_exhaustive([row, masked](int i) { return masked(row[i], i); }, v, mx, amax, temp, tk, tp, u, ztot, cnt_above, mass_above,
+                                     kmin, kmax);
     if (tid == 0) out[b] = id;
   };
+  u64 zl = 0, ztot;
   if (sbad || !isfinite(mx) || !isfinite(inv_t)) {
-    exhaustive();
+    each([&](float x, int) { zl += mass(x); });
+    block_scan_u64(zl, sm.wt, ztot);
+    exhaustive(ztot, 0, 0ull, 0u, ~0u);
     return;
   }
-  auto mass = [&](float x) { return fx(expf((x - mx) * inv_t)); };
   auto entry = [](uint32_t key, int id) { return (u64)key << 32 | (0xffffffffu - (uint32_t)id); };   // larger: earlier in the order
   const int k_limit = tk > 0 ? tk : 0x7fffffff;
   const bool keep_all = tk <= 0 && tp >= 1.f, few = tk > 0 && tk <= kTopList;
-  u64 zl = 0, ztot;
-  u64 last = 0;              // the last kept entry: kept are those not below it
+  u64 last = 0;              // the last kept entry with a mass: kept are those not below it, and some without a mass
   bool none = false;         // top_p leaves nothing
+  uint32_t kmin = ~0u, kmax = 0;
+  auto listed = [&](float x, int i) {
+    const uint32_t key = okey(x);
+    const int at = atomicAdd(&sm.n, 1);
+    if (at < kList) sm.list[at] = entry(key, i);
+    kmin = min(kmin, key), kmax = max(kmax, key);
+  };
   if (few) {
     // at least k of the threads' maxima, so at least k values, are not below their k-th
     sm.list[tid] = (u64)okey(own) << 32 | (uint32_t)tid;
@@ -334,12 +347,9 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
     const uint32_t bound = (uint32_t)(sm.list[tk - 1] >> 32);
     __syncthreads();
     each([&](float x, int i) {
-      zl += mass(x);
-      const uint32_t key = okey(x);
-      if (key >= bound) {
-        const int at = atomicAdd(&sm.n, 1);
-        if (at < kList) sm.list[at] = entry(key, i);
-      }
+      const u64 m = mass(x);
+      zl += m;
+      if (okey(x) >= bound && m > 0) listed(x, i);
     });
   } else if (keep_all) {
     each([&](float x, int) { zl += mass(x); });
@@ -389,11 +399,10 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
   } else if (!few) {
     each([&](float x, int i) {
       const int bin = min(__float2int_rz(fminf((mx - x) * inv_t, 1e6f) * 64.f), kBins - 1);
-      if (bin < bin_last) own_mass += mass(x);
-      if (bin == bin_last) {
-        const int at = atomicAdd(&sm.n, 1);
-        if (at < kList) sm.list[at] = entry(okey(x), i);
-      }
+      if (bin > bin_last) return;
+      const u64 m = mass(x);
+      if (bin < bin_last) own_mass += m;
+      else if (m > 0) listed(x, i);
     });
   }
 #pragma unroll
@@ -402,7 +411,10 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
   __syncthreads();
   const int n = sm.n;
   if (n > kList) {
-    exhaustive();
+    kmin = __reduce_min_sync(0xffffffffu, kmin), kmax = __reduce_max_sync(0xffffffffu, kmax);
+    if (lane == 0) atomicMin(&sm.kmin, kmin), atomicMax(&sm.kmax, kmax);
+    __syncthreads();
+    exhaustive(ztot, cnt_above, mass_above, sm.kmin, sm.kmax);
     return;
   }
   if (n > 0) {
