@@ -118,48 +118,22 @@ __global__ void __launch_bounds__(192, 1) gemm_prefill_kernel(const __grid_const
         uint32_t r[32];
         tmem_ld_32x32(d0 + c, r);
         tmem_ld_wait();
-        if (row >= g.M) continue;
-        float v[32];
+        if (row < g.M) {
+          float v[32];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-        if (gated) {
-          gate_block(v, g.act, g.limit);
-          st_f16x(dst + c / 2, v);
-          continue;
-        }
-        if (g.act) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = gemm_act(v[j], g.act);
-        }
-        if (vec && cols - c >= 32) {
-          if (g.accumulate) {
-            float4 o[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = ld_f4(dst + c + 4 * j);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[4 * j] += o[j].x, v[4 * j + 1] += o[j].y, v[4 * j + 2] += o[j].z, v[4 * j + 3] += o[j].w;
-          }
-          if constexpr (sizeof(OutT) == 4) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) st_f4(dst + c + 4 * j, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+          if (gated) {
+            gate_block(v, g.act, g.limit);
+            st_f16x(dst + c / 2, v);
           } else {
+            if (g.act) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 u;
-              __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&u);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) p[e] = __floats2bfloat162_rn(v[8 * j + 2 * e], v[8 * j + 2 * e + 1]);
-              reinterpret_cast<uint4*>(dst + c)[j] = u;
+              for (int j = 0; j < 32; ++j) v[j] = gemm_act(v[j], g.act);
             }
+            st_row32(dst + c, v, cols - c, vec, g.accumulate);
           }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (c + j < cols) {
-              if (g.accumulate) v[j] += ld_f(dst + c + j);
-              st_f(dst + c + j, v[j]);
-            }
         }
+        __syncwarp();      // the next columns are loaded by the warp as a whole
       }
       tc_fence_before();
       __syncwarp();

@@ -97,6 +97,28 @@ __device__ __forceinline__ void st_f16x(float* dst, const float* v) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) st_f4(dst + 4 * i, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
 }
+// 32 sums of a row (`left` of its columns exist from here on), added to what dst holds or stored as they are.  vec: dst starts on 16 bytes.
+template <typename OutT>
+__device__ __forceinline__ void st_row32(OutT* dst, float (&v)[32], int left, bool vec, bool accumulate) {
+  if (vec && left >= 32) {
+    if (accumulate) {
+      float4 o[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = ld_f4(dst + 4 * j);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[4 * j] += o[j].x, v[4 * j + 1] += o[j].y, v[4 * j + 2] += o[j].z, v[4 * j + 3] += o[j].w;
+    }
+    st_f16x(dst, v);
+    st_f16x(dst + 16, v + 16);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < left) {
+        if (accumulate) v[j] += ld_f(dst + j);
+        st_f(dst + j, v[j]);
+      }
+  }
+}
 
 // First and last row of a request's rows in the batch: rows of a request stand together at consecutive positions.
 __device__ __forceinline__ bool seg_first(const int* slots, const int* pos, int t) {

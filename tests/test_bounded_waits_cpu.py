@@ -1,4 +1,4 @@
-"""Kernels with bounded waits end after a wait that ran out: no warp is left at a barrier that another does not come to.
+"""Kernels with bounded waits: after one that ran out no warp is left at a barrier that another does not come to, and warps stay together.
 
 Read from the sources: such a wait runs out only when something else is broken, which no test brings about on a GPU."""
 import re
@@ -44,3 +44,13 @@ def test_no_barrier_in_a_loop_that_some_warps_leave(path):
             assert not re.search(r"\bok\b", header), where
             assert not re.search(r"\b(?:break|return)\b", src[first:last]), where
             assert not re.search(r"(?:!\s*ok|mbar_wait)\b[^;{}]*\)\s*\{?\s*continue\b", src[first:bar.start()]), where
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.stem)
+def test_lanes_without_a_row_come_to_the_next_load(path):
+    """Loads from tensor memory take a warp as a whole: where a loop issues them, no lane goes on to the next round ahead of the others."""
+    src = _source(path)
+    for header, first, last in _loops(src):
+        body = src[first:last]
+        if "tmem_ld_32x" in body and not any(first < f < last and "tmem_ld_32x" in src[f:e] for _, f, e in _loops(src)):
+            assert not re.search(r"\bcontinue\b", body[body.index("tmem_ld_32x"):]), f"{path.name}: for ({header.strip()})"
