@@ -70,9 +70,9 @@ __device__ __forceinline__ int sf_offset(int n, int kb) { return (n & 31) * 16 +
 
 // xq[2 pos] = hi row, xq[2 pos + 1] = lo row of token t for every route of t, pos = route_pos[t * topk + k]; the block exponents go
 // into the scale block of the position's route tile: sf[tile][K / 128][512] at rows 2 n and 2 n + 1, n = pos - tile start.
-// A CTA per token: its row is read and split once, for all of its routes.  8 192 tokens of six routes: 133 us, 227 us with a CTA per
-// route.
-constexpr int kMaxTopk = 128;     // a thread per route
+// A CTA per token and up to 128 of its routes: the row is read and split once for all of them.  8 192 tokens of six routes: 133 us,
+// 227 us with a CTA per route.
+constexpr int kRoutesAtOnce = 128;     // a thread per route
 __global__ void __launch_bounds__(128) moe_mx_permute_kernel(const __nv_bfloat16* __restrict__ x,
                                                              uint8_t* __restrict__ xq, uint8_t* __restrict__ sf,
                                                              const MxPlanHeader* __restrict__ hdr,
@@ -84,10 +84,11 @@ __global__ void __launch_bounds__(128) moe_mx_permute_kernel(const __nv_bfloat16
     if (threadIdx.x == 0) dsv4_set_error(DSV4_ERR_BAD_INDEX, 31, hdr->num_tiles);
     return;
   }
-  __shared__ int s_pos[kMaxTopk], s_tile[kMaxTopk], s_n[kMaxTopk];
-  const int tok = blockIdx.x;
-  if (threadIdx.x < topk) {
-    const int pos = route_pos[tok * topk + threadIdx.x];
+  __shared__ int s_pos[kRoutesAtOnce], s_tile[kRoutesAtOnce], s_n[kRoutesAtOnce];
+  const int tok = blockIdx.x, k0 = blockIdx.y * kRoutesAtOnce, first = tok * topk + k0;
+  const int nk = min(min(kRoutesAtOnce, topk - k0), routes - first);     // the last token may have fewer
+  if ((int)threadIdx.x < nk) {
+    const int pos = route_pos[first + threadIdx.x];
     int keep = -1, tile = 0, n = 0;
     if (pos >= 0 && pos < hdr->num_routes_local) {
       int lo = 0, hi = hdr->num_tiles - 1;   // the last tile that starts at or before pos (tiles are in position order)
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(128) moe_mx_permute_kernel(const __nv_bfloat16
       wh[i >> 2] |= hb << (8 * (i & 3));
       wl[i >> 2] |= lb << (8 * (i & 3));
     }
-    for (int k = 0; k < topk; ++k) {
+    for (int k = 0; k < nk; ++k) {
       const int pos = s_pos[k], n = s_n[k];
       if (pos < 0) continue;
       uint4* dh = reinterpret_cast<uint4*>(xq + (size_t)(2 * pos) * h + blk * 32);
@@ -474,12 +475,13 @@ int launch_mx_gemm(const void* w, const uint8_t* sfa, const void* xq, const uint
 DSV4_API int dsv4_moe_mx_permute(const void* x, void* xq, void* sf, const int* plan, int routes, int max_tiles, int topk,
                                  int h, int nt, cudaStream_t st) {
   if (routes <= 0) return 0;
-  if (h % 128 || (nt != 8 && nt != 16 && nt != 32 && nt != 64) || topk < 1 || topk > kMaxTopk || routes % topk) return 240;
+  if (h % 128 || (nt != 8 && nt != 16 && nt != 32 && nt != 64) || topk < 1) return 240;
   const MxPlanHeader* hdr = reinterpret_cast<const MxPlanHeader*>(plan);
   const int* tiles = plan + 4;
   const int* route_pos = tiles + 3 * max_tiles + routes;
-  dsv4_launch(moe_mx_permute_kernel, routes / topk, 128, 0, st, (const __nv_bfloat16*)x, (uint8_t*)xq, (uint8_t*)sf, hdr, tiles,
-              route_pos, topk, h, routes, max_tiles, nt);
+  const dim3 grid((routes + topk - 1) / topk, (topk + kRoutesAtOnce - 1) / kRoutesAtOnce);
+  dsv4_launch(moe_mx_permute_kernel, grid, 128, 0, st, (const __nv_bfloat16*)x, (uint8_t*)xq, (uint8_t*)sf, hdr, tiles, route_pos, topk,
+              h, routes, max_tiles, nt);
   return (int)cudaGetLastError();
 }
 
