@@ -35,13 +35,13 @@ HOST_LIB = HERE / "libdsv4_host.so"
 
 # sources (csrc/<name>.cu) a model family's forward pass and sampling need
 KERNEL_SETS = {
-    "layered": ("common", "comm", "elementwise", "sampling", "gemm_tcgen05", "gemm_rows", "gemm_prefill", "gemm_simt", "moe", "moe_bf16",
+    "layered": ("common", "comm", "elementwise", "sampling", "gemm_tcgen05", "gemm_rows", "gemm_prefill", "gemm_prefill_fp8", "gemm_simt", "moe", "moe_bf16",
                 "residual", "latent_attn", "flash_attn", "wkv", "wkv_chunk"),
-    "grouped": ("common", "comm", "elementwise", "sampling", "gemm_tcgen05", "gemm_rows", "gemm_prefill", "gemm_simt", "residual",
+    "grouped": ("common", "comm", "elementwise", "sampling", "gemm_tcgen05", "gemm_rows", "gemm_prefill", "gemm_prefill_fp8", "gemm_simt", "residual",
                 "grouped_attn", "flash_attn", "delta", "delta_chunk"),
-    "streams": ("common", "comm", "elementwise", "sampling", "gemm_tcgen05", "gemm_rows", "gemm_prefill", "gemm_simt", "moe", "moe_bf16",
+    "streams": ("common", "comm", "elementwise", "sampling", "gemm_tcgen05", "gemm_rows", "gemm_prefill", "gemm_prefill_fp8", "gemm_simt", "moe", "moe_bf16",
                 "residual", "streams", "grouped_attn", "flash_attn", "gla", "gla_chunk"),
-    "windows": ("common", "comm", "elementwise", "sampling", "gemm_tcgen05", "gemm_rows", "gemm_prefill", "gemm_simt", "residual",
+    "windows": ("common", "comm", "elementwise", "sampling", "gemm_tcgen05", "gemm_rows", "gemm_prefill", "gemm_prefill_fp8", "gemm_simt", "residual",
                 "grouped_attn", "latent_attn", "flash_attn", "mingru"),
 }
 
