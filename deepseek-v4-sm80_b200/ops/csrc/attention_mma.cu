@@ -43,7 +43,7 @@ struct TcSmem {
   uint8_t ones[1024];           // an 8-row group of ones; every group of the operand is this one
   float wmax[8][32], ref[8][32], mul[8][32];
   const __nv_bfloat16* rows[2][KT];     // cache rows of a tile's keys, null if masked
-  uint64_t full[4], empty[4], s_full, p_full, o_full;
+  uint64_t full[4], empty[4], s_full, p_full, o_full, drain;
   uint32_t tmem;
   int abort_flag;
 };
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_mma_kernel(const Attn
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 4; ++i) mbar_init(&sm.full[i], 1), mbar_init(&sm.empty[i], 1);
-    mbar_init(&sm.s_full, 1), mbar_init(&sm.p_full, 8), mbar_init(&sm.o_full, 1);
+    mbar_init(&sm.s_full, 1), mbar_init(&sm.p_full, 8), mbar_init(&sm.o_full, 1), mbar_init(&sm.drain, 1);
     sm.abort_flag = 0;
     mbar_fence_init();
   }
@@ -383,10 +383,10 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_mma_kernel(const Attn
   }
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag && warp == 8 && lane == 0)
-    for (int i = 0; i < 100; ++i) __nanosleep(1000);      // after a wait that ran out: what is in flight retires
-  __syncthreads();
-  if (warp == 8) tmem_dealloc(tmem, 512);
+  if (warp == 8) {
+    if (*abort_flag) drain_after_abort(&sm.drain, elect_one());
+    tmem_dealloc(tmem, 512);
+  }
 }
 
 // out[t][head] = sum_s acc_s 2^(ref_s - M) / sum_s l_s 2^(ref_s - M); one warp per head, 16 dims a lane.

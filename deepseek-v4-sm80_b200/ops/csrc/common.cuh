@@ -198,6 +198,18 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
+// After a bounded wait that ran out, behind the last barrier of the CTA and ahead of tmem_dealloc: the MMAs issued so far retire and the
+// copies in flight land, each with a limit (2 ms, 100 us).  The issuing warp as a whole; issuer: the thread that issued;  drain: a barrier
+// for one arrival per issuing thread that nothing else uses.
+__device__ __forceinline__ void drain_after_abort(uint64_t* drain, bool issuer) {
+  if (issuer) {
+    umma_commit(drain);
+    for (int i = 0; i < 20000 && !mbar_try_wait(drain, 0); ++i) __nanosleep(100);
+    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  }
+  __syncwarp();
+  tc_fence_after();
+}
 
 // D[tmem] (+)= A[smem] * B[smem];  kind::f16 covers fp16/bf16 inputs, kind::f8f6f4 the 8/6/4-bit float inputs
 __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,

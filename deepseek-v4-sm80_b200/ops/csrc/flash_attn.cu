@@ -46,7 +46,7 @@ struct FlashArgs {
 };
 
 struct FlashBars {
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], o_full[2];
+  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], o_full[2], drain;
   uint32_t tmem;
   int abort_flag;
 };
@@ -80,7 +80,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int head = blockIdx.x, kv_head = head / a.group;
 
   if (threadIdx.x == 0) {
-    mbar_init(&b->q_full, 1);
+    mbar_init(&b->q_full, 1), mbar_init(&b->drain, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&b->k_full[i], 1), mbar_init(&b->k_empty[i], 1);
       mbar_init(&b->v_full[i], 1), mbar_init(&b->v_empty[i], 1);
@@ -395,7 +395,10 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, 512);
+  if (warp == 1) {
+    if (*abort_flag) drain_after_abort(&b->drain, elect_one());
+    tmem_dealloc(tmem, 512);
+  }
 }
 
 template <int NB, int MODE>

@@ -39,13 +39,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_prefill_fp8_kernel(const __g
   extern __shared__ uint8_t fsm_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fsm_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * kPad);
-  uint64_t *empty = full + kStages, *tfull = empty + kStages, *tempty = tfull + 2;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty + 2);
+  uint64_t *empty = full + kStages, *tfull = empty + kStages, *tempty = tfull + 2, *drain = tempty + 2;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) mbar_init(&full[i], 5), mbar_init(&empty[i], 1);    // the copies and four warps of scales
     for (int i = 0; i < 2; ++i) mbar_init(&tfull[i], 1), mbar_init(&tempty[i], 4);
+    mbar_init(drain, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmA);
@@ -179,7 +180,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_prefill_fp8_kernel(const __g
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, 512);
+  if (warp == 1) {
+    if (*abort_flag) drain_after_abort(drain, elect_one());
+    tmem_dealloc(tmem, 512);
+  }
 }
 
 template <typename OutT>

@@ -127,7 +127,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint8_t* sf_all = smem + S * Cfg::kStageBytes;  // fp8: [nkt] row-scale blocks, then the block of ones
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * Cfg::kStageBytes + Cfg::kSfBytes);
   uint64_t* empty = full + S;
-  uint64_t* tfull = empty + S;   // [8]
+  uint64_t* tfull = empty + S;   // [8]; the last one: drain
   uint64_t* tempty = tfull + 8;  // [8]
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
@@ -541,7 +541,10 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
+  if (warp == 1) {
+    if (*abort_flag) drain_after_abort(&tfull[7], elect_one());
+    tmem_dealloc(tmem_base, kTmemCols);
+  }
 }
 
 struct LaunchOpts {

@@ -66,7 +66,8 @@ indexer_logits_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_
   uint64_t* tfull = empty + SA;    // [2]
   uint64_t* tempty = tfull + 2;    // [2]
   uint64_t* qfull = tempty + 2;    // [1]
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(qfull + 1);
+  uint64_t* drain = qfull + 1;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -78,7 +79,7 @@ indexer_logits_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
     for (int i = 0; i < 2; ++i) mbar_init(&tfull[i], 1), mbar_init(&tempty[i], 32 * EW);
-    mbar_init(qfull, 1);
+    mbar_init(qfull, 1), mbar_init(drain, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmK);
@@ -274,7 +275,10 @@ indexer_logits_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, (uint32_t)a.tmem_cols);
+  if (warp == 1) {
+    if (*abort_flag) drain_after_abort(drain, elect_one());
+    tmem_dealloc(tmem_base, (uint32_t)a.tmem_cols);
+  }
 }
 
 }  // namespace

@@ -383,7 +383,8 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   uint64_t* tfull = oempty + kOBufs;    // [2]         accumulators complete (one commit per issuer)
   uint64_t* tempty = tfull + 2;         // [2]         accumulators drained by the epilogue
   uint64_t* xfull = tempty + 2;         // [2]         GEMM1: the up warps' sums are in the exchange buffer
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(xfull + 2);
+  uint64_t* drain = xfull + 2;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -397,6 +398,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     for (int i = 0; i < kOBufs; ++i)
       mbar_init(&ofull[i], kBuilders / 64 + 1), mbar_init(&oempty[i], 1);
     for (int i = 0; i < 2; ++i) mbar_init(&tfull[i], kDual ? 2 : 1), mbar_init(&tempty[i], 4), mbar_init(&xfull[i], 2);
+    mbar_init(drain, kDual ? 2 : 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmW);
@@ -647,7 +649,11 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, S::kTmemCols);
+  if (kDual && warp == kIssuerWarp1 && lane == 0 && *abort_flag) umma_commit(drain);
+  if (warp == 1) {
+    if (*abort_flag) drain_after_abort(drain, lane == 0);
+    tmem_dealloc(tmem_base, S::kTmemCols);
+  }
 }
 
 // out[t] = bf16( float(bf16(sum_k local route rows)) + float(shared[t]) ); rows >= num_valid -> 0

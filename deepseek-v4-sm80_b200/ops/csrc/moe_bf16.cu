@@ -60,8 +60,8 @@ __global__ void __launch_bounds__(192, 1) moe_bf16_gemm_kernel(const __grid_cons
   extern __shared__ uint8_t gsm_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * C::kStageBytes);
-  uint64_t *empty = full + S, *tfull = empty + S, *tempty = tfull + 2;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty + 2);
+  uint64_t *empty = full + S, *tfull = empty + S, *tempty = tfull + 2, *drain = tempty + 2;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(192, 1) moe_bf16_gemm_kernel(const __grid_cons
       mbar_init(&empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) mbar_init(&tfull[i], 1), mbar_init(&tempty[i], 4);
+    mbar_init(drain, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmA);
@@ -178,7 +179,10 @@ __global__ void __launch_bounds__(192, 1) moe_bf16_gemm_kernel(const __grid_cons
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, C::kCols);
+  if (warp == 1) {
+    if (*abort_flag) drain_after_abort(drain, lane == 0);
+    tmem_dealloc(tmem, C::kCols);
+  }
 }
 
 // xs[pos] = x[sorted_route[pos] / topk], rows of d8 16-byte pieces

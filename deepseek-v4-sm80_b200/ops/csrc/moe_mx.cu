@@ -429,19 +429,10 @@ moe_mx_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   }
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag) {
-    // a wait ran out (the status word says where): before the tensor memory is freed and the CTA leaves, let the
-    // MMAs already issued retire and the copies in flight land, each with a limit of its own
-    if (warp == 1 && elect_one()) {
-      umma_commit(drain);
-      for (int i = 0; i < 20000 && !mbar_try_wait(drain, 0); ++i) __nanosleep(100);
-    }
-    if (threadIdx.x == 0)
-      for (int i = 0; i < 100; ++i) __nanosleep(1000);
-    tc_fence_before();
-    __syncthreads();
+  if (warp == 1) {
+    if (*abort_flag) drain_after_abort(drain, elect_one());
+    tmem_dealloc(tmem_base, S::kTmemCols);
   }
-  if (warp == 1) tmem_dealloc(tmem_base, S::kTmemCols);
 }
 
 template <int MODE, int NT>

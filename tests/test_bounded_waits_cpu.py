@@ -54,3 +54,11 @@ def test_lanes_without_a_row_come_to_the_next_load(path):
         body = src[first:last]
         if "tmem_ld_32x" in body and not any(first < f < last and "tmem_ld_32x" in src[f:e] for _, f, e in _loops(src)):
             assert not re.search(r"\bcontinue\b", body[body.index("tmem_ld_32x"):]), f"{path.name}: for ({header.strip()})"
+
+
+@pytest.mark.parametrize("path", [p for p in SOURCES if "tmem_dealloc" in p.read_text()], ids=lambda p: p.stem)
+def test_tensor_memory_is_freed_behind_what_is_in_flight(path):
+    """After a wait that ran out, MMAs and copies may still be under way: they are waited for, with a limit, before tensor memory is freed."""
+    src = _source(path)
+    for free in re.finditer(r"tmem_dealloc\(", src):
+        assert re.search(r"if \(\*abort_flag\) drain_after_abort\([^;]*;\s*$", src[:free.start()]), path.name
