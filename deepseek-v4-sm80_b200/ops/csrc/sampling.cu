@@ -333,23 +333,22 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
   const bool keep_all = tk <= 0 && tp >= 1.f, few = tk > 0 && tk <= kTopList;
   u64 last = 0;              // the last kept entry with a mass: kept are those not below it, and some without a mass
   bool none = false;         // top_p leaves nothing
-  uint32_t kmin = ~0u, kmax = 0;
-  auto listed = [&](float x, int i) {
-    const uint32_t key = okey(x);
+  auto listed = [&](uint32_t key, int i) {
     const int at = atomicAdd(&sm.n, 1);
     if (at < kList) sm.list[at] = entry(key, i);
-    kmin = min(kmin, key), kmax = max(kmax, key);
   };
+  uint32_t bound = 0;
   if (few) {
     // at least k of the threads' maxima, so at least k values, are not below their k-th
     sm.list[tid] = (u64)okey(own) << 32 | (uint32_t)tid;
     sort_list(sm.list, 1024);
-    const uint32_t bound = (uint32_t)(sm.list[tk - 1] >> 32);
+    bound = (uint32_t)(sm.list[tk - 1] >> 32);
     __syncthreads();
     each([&](float x, int i) {
       const u64 m = mass(x);
       zl += m;
-      if (okey(x) >= bound && m > 0) listed(x, i);
+      const uint32_t key = okey(x);
+      if (key >= bound && m > 0) listed(key, i);
     });
   } else if (keep_all) {
     each([&](float x, int) { zl += mass(x); });
@@ -402,7 +401,7 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
       if (bin > bin_last) return;
       const u64 m = mass(x);
       if (bin < bin_last) own_mass += m;
-      else if (m > 0) listed(x, i);
+      else if (m > 0) listed(okey(x), i);
     });
   }
 #pragma unroll
@@ -411,6 +410,12 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
   __syncthreads();
   const int n = sm.n;
   if (n > kList) {
+    uint32_t kmin = ~0u, kmax = 0;
+    each([&](float x, int) {
+      const uint32_t key = okey(x);
+      const int bin = min(__float2int_rz(fminf((mx - x) * inv_t, 1e6f) * 64.f), kBins - 1);
+      if ((few ? key >= bound : bin == bin_last) && mass(x) > 0) kmin = min(kmin, key), kmax = max(kmax, key);
+    });
     kmin = __reduce_min_sync(0xffffffffu, kmin), kmax = __reduce_max_sync(0xffffffffu, kmax);
     if (lane == 0) atomicMin(&sm.kmin, kmin), atomicMax(&sm.kmax, kmax);
     __syncthreads();
