@@ -1,11 +1,14 @@
-// Projections of a few rows (decode of a few requests):  out[M,N] = X[M,K] W[N,K]^T  for M <= 24, bf16 or e4m3 with power-of-two
-// block scales (as in gemm_tcgen05.cu).  Weights are read once and that is the time: 33.5 MB take 5.2 us at the HBM rate.
+// Projections of a few rows (decode of a few requests):  out[M,N] = X[M,K] W[N,K]^T  for M <= 24 in bf16 or M <= 16 in e4m3 with
+// power-of-two block scales (as in gemm_tcgen05.cu); ops/gemm.py (few_rows) says which sizes come here.  Weights are read once and that
+// is the time: 33.5 MB take 5.2 us at the HBM rate.
 //
 // One CTA per output tile with tensor memory, a TMA ring and a cluster reduction (gemm_tcgen05.cu) spends most of its life starting and
 // ending at this size.  Here a warp loads 16 weight rows straight into registers, 16 bytes a lane, as the A operand of
 // mma.sync m16n8k16 (rows of X are the 8 columns), one batch of loads ahead of the products; the 8 warps of a CTA share K between
 // them as far as the output leaves SMs idle, and add their sums in order in shared memory.  Nothing waits on anything else before that.
-// The projections of an attention block (161 MB of weights): one row 54 us, 14 rows 65, 24 rows 87; tiled 94 to 97 at each.
+// The first 8 columns are nearly free (4 096 x 4 096 in bf16: 8.1 us for one row, 8.7 for eight, 10.8 for 24; 28 to 19 in tiles).
+// e4m3 has conversions in front of each product, which with 16 rows outweigh what tiles cost from about 8 192 weight rows on
+// (32 768 x 1 024: 12.7 us for one row, 18.2 for 16; 15 in tiles).
 //
 // A lane's 16 bytes are consecutive places of K of one weight row, and the same places of one row of X: the order of the contraction
 // is free as long as both operands agree.  e4m3 becomes f16 exactly, a product of two fits fp32, and every 128 places the fp32 sum is
@@ -163,9 +166,9 @@ int launch(const RowsArgs& a, int batches, cudaStream_t st) {
   const dim3 grid((a.N + per_cta - 1) / per_cta, batches);
   if (a.M <= 8)
     dsv4_launch(gemm_rows_kernel<1, FP8, OutT>, grid, kWarps * 32, 0, st, a);
-  else if (a.M <= 16)
+  else if (FP8 || a.M <= 16)
     dsv4_launch(gemm_rows_kernel<2, FP8, OutT>, grid, kWarps * 32, 0, st, a);
-  else
+  else if constexpr (!FP8)
     dsv4_launch(gemm_rows_kernel<3, FP8, OutT>, grid, kWarps * 32, 0, st, a);
   return (int)cudaGetLastError();
 }
@@ -193,7 +196,7 @@ DSV4_API int dsv4_gemm_rows_bf16(const void* x, const void* w, void* out, int M,
 DSV4_API int dsv4_gemm_rows_fp8(const void* x, const void* w, void* out, const float* sa, const float* sb, int M, int N, int K, int ldx,
                                 int ldw, int ldo, int out_fp32, int accumulate, cudaStream_t st) {
   if (M <= 0 || N <= 0) return 0;
-  if (M > 24 || K <= 0 || K % 128 || ldx % 16 || ldw % 16 || (((uintptr_t)x | (uintptr_t)w) & 15)) return 681;
+  if (M > 16 || K <= 0 || K % 128 || ldx % 16 || ldw % 16 || (((uintptr_t)x | (uintptr_t)w) & 15)) return 681;
   const RowsArgs a{(const uint8_t*)x, (const uint8_t*)w, out, sa, sb, M, N, K, ldx, ldw, ldo, share_k(N, 1, K / 64), accumulate,
                    dsv4_weight_prefetch()};
   return out_fp32 ? launch<true, float>(a, 1, st) : launch<true, __nv_bfloat16>(a, 1, st);

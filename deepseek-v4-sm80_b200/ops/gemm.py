@@ -142,7 +142,7 @@ def gemm_bf16(x, w, out=None, out_dtype=torch.bfloat16, accumulate=False, bn=0, 
                 I(o2.stride(0)), I(1 if out.dtype == torch.float32 else 0), I(1 if accumulate else 0), I(ACTS[act]), F(0.0), I(1),
                 I(NUM_SMS_HINT))
         return out
-    if bn == 0 and splits == 0 and act is None and _few_rows(x2, w, m, k, 32):
+    if bn == 0 and splits == 0 and act is None and _few_rows(x2, w, m, n, k, 1, 32):
         nv.call("gemm_rows_bf16", nv.ptr(x2), nv.ptr(w), nv.ptr(o2), I(m), I(n), I(k), I(x2.stride(0)), I(w.stride(0)),
                 I(o2.stride(0)), I(1 if out.dtype == torch.float32 else 0), I(1 if accumulate else 0), I(1))
         return out
@@ -175,15 +175,31 @@ def _many_rows(x2, w, m: int, n: int, k: int, groups: int) -> bool:
     return prefill_tiles(m, n, groups) >= PREFILL_MIN_TILES and _tma_ok(x2, w, k)
 
 
-# Rows up to which the kernel without tiles (csrc/gemm_rows.cu) is the faster one: its work grows by the eight rows, the tiled kernel's
-# does not up to 128.  The projections of an attention block take 87 us there at 24 rows, 102 at 30, and 95 in tiles.
-FEW_ROWS = 24
+def few_rows(m: int, n: int, k: int, groups: int = 1, fp8: bool = False) -> bool:
+    """Whether a projection of these sizes runs on the kernel without tiles (csrc/gemm_rows.cu) instead of tiles of 128 rows, whose time does
+    not depend on m.  Its work grows by the eight rows.  Times below in us, without tiles / with them, of a projection and the kernel that
+    makes its input, weights from HBM."""
+    if m <= 8:
+        # fp8 1 536 x 4 096: 6.9 / 10.0, 32 768 x 1 024: 15.0 / 17.5, 4 096 x 256: 4.9 / 5.1; bf16 129 280 x 4 096: 189 / 307
+        return m > 0
+    if fp8:
+        # Each e4m3 weight becomes f16 in the kernel, which takes the time when there are two or three groups of rows.  16 rows of
+        # 4 096 x 4 096: 11.2 / 13.0, 4 096 x 512: 6.0 / 6.1; 4 096 x 256: 6.4 / 5.2.  Tiles win where they fill the GPU (12 rows of
+        # 32 768 x 1 024: 18.3 / 17.5), but only alone: beside the compressor's branch, which they leave no shared memory, the attention block
+        # of 12 requests takes 90 / 98 in all.  With 17 requests it is 105 / 105, and 96 / 86 in a layer without that branch.
+        return m <= 16 and k >= 512
+    if m < 16:
+        # 15 rows of 4 096 x 4 096: 11.5 / 31.0, 129 280 x 4 096: 233 / 318; 8 x (4 096 -> 2 048): 34.9 / 32.9, 4 096 x 128: 5.4 / 5.0
+        return k >= 256 and (groups == 1 or groups * n <= 8192)
+    # 24 rows of 4 096 x 4 096: 12.9 / 21.2, 8 192 x 4 096: 22.6 / 22.5; 16 rows of 129 280 x 4 096: 233 / 200, 12 480 x 4 096: 32.9 / 27.5;
+    # 20 rows of 1 024 x 16 384: 25.7 / 24.3, 256 x 256: 5.1 / 4.9
+    return m <= 24 and 512 <= k <= 8192 and groups * n <= 8192
 
 
-def _few_rows(x2, w, m: int, k: int, whole: int) -> bool:
+def _few_rows(x2, w, m: int, n: int, k: int, groups: int, whole: int) -> bool:
     """Whether the kernel for a few rows takes this projection: K in multiples of `whole`, rows on 16 bytes."""
     e = x2.element_size()
-    return (0 < m <= FEW_ROWS and k % whole == 0 and x2.stride(0) * e % 16 == 0 and w.stride(0) * e % 16 == 0
+    return (few_rows(m, n, k, groups, e == 1) and k % whole == 0 and x2.stride(0) * e % 16 == 0 and w.stride(0) * e % 16 == 0
             and x2.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
@@ -286,7 +302,7 @@ def gemm_bf16_grouped(x, w, groups: int, out=None):
         nv.call("gemm_prefill", nv.ptr(x), nv.ptr(w), nv.ptr(out), I(t), I(n), I(k), I(x.stride(0)), I(w.stride(0)),
                 I(out.stride(0)), I(0), I(0), I(0), F(0.0), I(groups), I(NUM_SMS_HINT))
         return out
-    if _few_rows(x, w, t, k, 32):
+    if _few_rows(x, w, t, n, k, groups, 32):
         nv.call("gemm_rows_bf16", nv.ptr(x), nv.ptr(w), nv.ptr(out), I(t), I(n), I(k), I(x.stride(0)), I(w.stride(0)), I(out.stride(0)),
                 I(1 if out.dtype == torch.float32 else 0), I(0), I(groups))
         return out
@@ -323,7 +339,7 @@ def gemm_fp8(xq, sx, wq, sw, out=None, out_dtype=torch.bfloat16, accumulate=Fals
                 I(wq.stride(0)), I(o2.stride(0)), I(1 if out.dtype == torch.float32 else 0), I(1 if accumulate else 0),
                 I(NUM_SMS_HINT))
         return out
-    if bn == 0 and splits == 0 and _few_rows(x2, wq, m, k, 128):
+    if bn == 0 and splits == 0 and _few_rows(x2, wq, m, n, k, 1, 128):
         nv.call("gemm_rows_fp8", nv.ptr(x2), nv.ptr(wq), nv.ptr(o2), nv.ptr(s2), nv.ptr(sw), I(m), I(n), I(k), I(x2.stride(0)),
                 I(wq.stride(0)), I(o2.stride(0)), I(1 if out.dtype == torch.float32 else 0), I(1 if accumulate else 0))
         return out
