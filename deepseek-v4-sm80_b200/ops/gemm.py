@@ -137,7 +137,8 @@ def gemm_bf16(x, w, out=None, out_dtype=torch.bfloat16, accumulate=False, bn=0, 
         out = torch.empty(*x.shape[:-1], n, dtype=out_dtype, device=x.device)
     o2 = out.reshape(-1, n) if out.is_contiguous() else out
     assert o2.stride(-1) == 1
-    if bn == 0 and splits == 0 and act not in GATES and _many_rows(x2, w, m, n, k, 1):
+    if (bn == 0 and splits == 0 and act not in GATES and _many_rows(x2, w, m, n, k, 1) and fewer_waves(m, n)
+            and _rows_on_16(o2, n, 1)):
         nv.call("gemm_prefill", nv.ptr(x2), nv.ptr(w), nv.ptr(o2), I(m), I(n), I(k), I(x2.stride(0)), I(w.stride(0)),
                 I(o2.stride(0)), I(1 if out.dtype == torch.float32 else 0), I(1 if accumulate else 0), I(ACTS[act]), F(0.0), I(1),
                 I(NUM_SMS_HINT))
@@ -173,6 +174,28 @@ def prefill_tiles(m: int, n: int, groups: int) -> int:
 def _many_rows(x2, w, m: int, n: int, k: int, groups: int) -> bool:
     """Whether the persistent kernel takes this bf16 projection."""
     return prefill_tiles(m, n, groups) >= PREFILL_MIN_TILES and _tma_ok(x2, w, k)
+
+
+def fewer_waves(m: int, n: int, groups: int = 1, fp8: bool = False) -> bool:
+    """Whether the persistent kernels' wider tiles are the better split of a result over the SMs than tiles of 128 x 128.
+
+    bf16: a wave of 128 x 256 tiles takes about 7/6 of a wave of 128 x 128 ones (K = 4 096: 28, 50, 74, 98 us for one to four waves, and 26,
+    44, 64, 85), so it has to save waves.  6 363 rows of 256 x 4 096 columns: 34 / 45 us; 12 763 of 128 columns, half of each tile padding:
+    30 / 26; 9 563 of 264, one tile more than a wave: 49 / 44; 12 763 of 264: 52 / 63.
+    fp8: a wave costs the same, so from the second wave of small tiles on.  5 339 rows of 512 x 4 096: 17.5 / 32.0 us; 4 315, one wave in
+    both: 17.3 / 17.9, and with K = 512: 7.5 / 7.5; 3 163 rows of 640 x 512: 8.2 / 7.6."""
+    small = -(-m // 128) * -(-n // 128) * groups
+    if fp8:
+        return m > 128 and small > NUM_SMS_HINT
+    waves = lambda tiles: -(-tiles // NUM_SMS_HINT)  # noqa: E731
+    return 7 * waves(prefill_tiles(m, n, groups)) <= 6 * waves(small)
+
+
+def _rows_on_16(o2, n: int, groups: int) -> bool:
+    """Results whose rows (of every group) start on 16 bytes.  Others are stored value by value, which the four warps that the persistent
+    kernels have for it take longer over than the CTAs of small tiles do: 12 763 rows of 300 x 512 49 / 34 us in bf16, 37 / 32 in e4m3."""
+    e = o2.element_size()
+    return o2.data_ptr() % 16 == 0 and o2.stride(0) * e % 16 == 0 and (groups == 1 or n * e % 16 == 0)
 
 
 def few_rows(m: int, n: int, k: int, groups: int = 1, fp8: bool = False) -> bool:
@@ -298,7 +321,8 @@ def gemm_bf16_grouped(x, w, groups: int, out=None):
     assert x.is_contiguous() and w.is_contiguous() and x.dtype == torch.bfloat16
     if out is None:
         out = torch.empty(t, groups * n, dtype=x.dtype, device=x.device)
-    if out.dtype == torch.bfloat16 and _many_rows(x, w, t, n, k, groups):
+    if (out.dtype == torch.bfloat16 and _many_rows(x, w, t, n, k, groups) and fewer_waves(t, n, groups)
+            and _rows_on_16(out, n, groups)):
         nv.call("gemm_prefill", nv.ptr(x), nv.ptr(w), nv.ptr(out), I(t), I(n), I(k), I(x.stride(0)), I(w.stride(0)),
                 I(out.stride(0)), I(0), I(0), I(0), F(0.0), I(groups), I(NUM_SMS_HINT))
         return out
@@ -311,12 +335,6 @@ def gemm_bf16_grouped(x, w, groups: int, out=None):
     nv.call("gemm_bf16", nv.ptr(x), nv.ptr(w), nv.ptr(out), I(t), I(n), I(k), I(x.stride(0)), I(w.stride(0)),
             I(out.stride(0)), I(0), I(0), I(bn), I(groups), I(splits), nv.ptr(ws), nv.ptr(cnt), I(0), F(0.0))
     return out
-
-
-# 128 x 192 output tiles from which the persistent FP8 kernel (csrc/gemm_prefill_fp8.cu) fills the GPU: 8 192 rows of the four FP8
-# projections of an attention block (1 536 x 4 096, 32 768 x 1 024, 8 192 x 1 024, 4 096 x 8 192) take 815 us there and 1 653 us on one
-# CTA per 128 x 128 tile
-FP8_PREFILL_MIN_TILES = 100
 
 
 def gemm_fp8(xq, sx, wq, sw, out=None, out_dtype=torch.bfloat16, accumulate=False, bn=0, splits=0):
@@ -334,7 +352,9 @@ def gemm_fp8(xq, sx, wq, sw, out=None, out_dtype=torch.bfloat16, accumulate=Fals
     if out is None:
         out = torch.empty(*xq.shape[:-1], n, dtype=out_dtype, device=xq.device)
     o2 = out.reshape(-1, n)
-    if bn == 0 and splits == 0 and m > 128 and -(-m // 128) * -(-n // 192) >= FP8_PREFILL_MIN_TILES:
+    # 8 192 rows of the four FP8 projections of an attention block (1 536 x 4 096, 32 768 x 1 024, 8 192 x 1 024, 4 096 x 8 192) take
+    # 730 us on the persistent kernel (csrc/gemm_prefill_fp8.cu) and 1 653 us on one CTA per 128 x 128 tile
+    if bn == 0 and splits == 0 and fewer_waves(m, n, fp8=True) and _rows_on_16(o2, n, 1):
         nv.call("gemm_prefill_fp8", nv.ptr(x2), nv.ptr(wq), nv.ptr(o2), nv.ptr(s2), nv.ptr(sw), I(m), I(n), I(k), I(x2.stride(0)),
                 I(wq.stride(0)), I(o2.stride(0)), I(1 if out.dtype == torch.float32 else 0), I(1 if accumulate else 0),
                 I(NUM_SMS_HINT))
