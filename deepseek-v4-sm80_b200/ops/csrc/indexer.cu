@@ -119,7 +119,10 @@ constexpr int kTopList = 512;    // entries of the k-th one's part that are put 
 // finds the k-th key byte by byte instead.  The four passes read registers: V float4 a thread hold the row of up to NT * 4 * V
 // entries, a warp consecutive ones (V = 0: longer rows, read again by each pass).
 // Bound by the steps of one row, not by its bytes: rows in flight hide them (512 threads for the rows of prompts: three CTAs an SM).
-// 4 096 rows of about 7 700: 130 us, against 775 us with four passes over key bytes whose 256 counts one thread walked.
+// In us, against four passes over key bytes whose 256 counts one thread walked: 4 096 rows of 8 192 normal scores 127 / 651, of equal ones
+// 253 / 877, with one far outlier 258 / 650; 2 048 rows of 32 768: 255 / 823, equal 573 / 897; 512 rows of 65 536: 153 / 419, equal
+// 298 / 452.  Rows with a score that is not finite, which end after the first pass, are the slower ones beyond 8 192 entries: 2 048 rows of
+// 32 768 73 / 53, 512 of 65 536 37 / 28.
 template <int NT, int V>
 __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_kernel(const float* __restrict__ logits, int width,
                                                   const int* __restrict__ pos, int* __restrict__ idx,
@@ -166,7 +169,14 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_kernel(const float
 #pragma unroll
       for (int u = 0; u < V; ++u) f(held[u], first + 128 * u);
     } else {
-      for (int i = 0; i < per && w * per + i < n; i += 128) f(load(first + i), first + i);
+      for (int i = 0; i < per && w * per + i < n; i += 512) {      // four loads in flight
+        float4 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = i + 128 * u < per ? load(first + i + 128 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (i + 128 * u < per && w * per + i + 128 * u < n) f(x[u], first + i + 128 * u);
+      }
     }
   };
   auto each = [&](auto f) {
