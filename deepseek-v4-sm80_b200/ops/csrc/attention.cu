@@ -2,10 +2,10 @@
 //   {sink} U {selected C4 rows | all C128 rows | nothing} U {sliding window rows},
 // keys and values being the same 512-d latent row (K = V), softmax scale 512^-1/2.
 //
-// One CTA per token.  Every gathered row is fetched once (cp.async into 128B-swizzled shared memory, double
-// buffered) and shared by all local heads; both contractions run on the tensor cores with warp-level
-// mma.sync.m16n8k16 (bf16 in, fp32 accumulate): with 8..64 heads per token the M extent is 16..64, far below the
-// 128-row tiles tcgen05 wants, and the kernel is bound by the row gather, so the warp-level shape is the better fit.
+// 8, 16 or 32 local heads (the shards of a layer; 64 heads: attention_mma.cu).  One CTA per token.  Every gathered row is
+// fetched once (cp.async into 128B-swizzled shared memory, double buffered) and shared by all local heads; both
+// contractions run on the tensor cores with warp-level mma.sync.m16n8k16 (bf16 in, fp32 accumulate).  tcgen05 would take
+// the heads as columns of instructions of 128 keys: with 8 to 32 of them most of what it reads for a key is not used.
 //   S phase : warp (mt, g) computes the 16 x 8 score tile of head tile mt and key group g (32 k-steps)
 //   softmax : online (m, l) per head, probabilities to shared memory as bf16
 //   PV phase: warp (mt, g) owns head tile mt and a 512/G slice of the output dims in registers
@@ -62,7 +62,7 @@ template <int HL>
 struct AttnCfg {
   static constexpr int HP = HL < 16 ? 16 : HL;          // padded head rows
   static constexpr int MT = HP / 16;                     // 16-row head tiles
-  static constexpr int NW = MT >= 4 ? 16 : 8;            // warps
+  static constexpr int NW = 8;                           // warps
   static constexpr int G = NW / MT;                      // warps per head tile
   static constexpr int KT = 8 * G;                       // keys per tile: one 16x8 score tile per warp
   static constexpr int DW = D / G;                       // output dims per warp

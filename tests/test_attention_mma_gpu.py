@@ -1,5 +1,5 @@
 """The tcgen05 form of the sparse latent attention (64 heads): several tokens per CTA, masked keys, padded rows, maxima that grow from
-tile to tile, splits without keys; and a 4:1 history attended whole, without a selection."""
+tile to tile, splits without keys; and a 4:1 history attended whole, without a selection, at every number of local heads."""
 import types
 
 import pytest
@@ -76,3 +76,18 @@ def test_a_whole_history_is_the_selection_of_all_its_entries():
     cpu, dev = (q, swa, swa_map, comp, sink), tuple(x.to(DEV) for x in (q, swa, swa_map, comp, sink))
     assert torch.equal(one(None, None, fb, *cpu), one(idx, n, fb, *cpu))
     assert torch.equal(one(None, None, _on(fb), *dev), one(idx.to(DEV), n.to(DEV), _on(fb), *dev))
+
+
+@pytest.mark.parametrize("heads", [8, 16, 32, 64])
+@pytest.mark.parametrize("t,prefill", [(1, False), (7, False), (200, True)])
+def test_whole_histories_of_sharded_heads(heads, t, prefill):
+    """4:1 entries without a list, in a layer's shards too: as many splits as the wrapper takes, and numbers that leave some without keys."""
+    from minisgl.ops import cuda
+
+    fb, swa, swa_map, comp, q, sink = _state(4, t, heads + t)
+    fb.is_prefill = prefill
+    q, sink = q[:, :heads].contiguous() * 6, sink[:heads].contiguous()
+    want = O.attention(q, fb, swa, swa_map, comp, 4, None, None, sink, D ** -0.5, PS, 128)
+    dev = [x.to(DEV) for x in (q, swa, swa_map, comp, sink)]
+    for ns in (0, 1, 3, 32):
+        _close(cuda.attention(dev[0], _on(fb), dev[1], dev[2], dev[3], 4, None, None, dev[4], D ** -0.5, PS, 128, nsplit=ns), want)
