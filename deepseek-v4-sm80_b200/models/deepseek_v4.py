@@ -106,7 +106,8 @@ class DSV4Model:
         iw = None
         qkv = None
         # a history of no more entries than are selected is attended whole: its queries and scores for a choice are not computed (the
-        # indexer's cache is written all the same, for later tokens)
+        # indexer's cache is written all the same, for later tokens).  No score is looked at, so one that is not finite, for which a
+        # selection leaves a token its window alone, drops nothing here.
         choose = ratio == 4 and fb.max_context // 4 > cfg.index_topk
         if sp is not None:
             # the all-gather is fused into this GEMM's loads; everything else that reads y is issued behind it

@@ -185,8 +185,8 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 // One lane of a converged warp.  A warp whose lanes all walk the issuer's loops, with only the instructions under this predicate, keeps
-// descriptors and addresses in uniform registers; in a branch that one lane takes they are moved there for every instruction
-// (128 x 64 x 16: 48 cycles each, which is what shared memory feeds, against 72 to 110).
+// descriptors and addresses in uniform registers; in a branch that one lane takes they are moved there for every instruction.  Four FP8
+// projections of 8 192 rows: 815 -> 730 us (gemm_prefill_fp8.cu); expert products of 128 tokens: 551 -> 494 us (moe_mx.cu).
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));

@@ -2,9 +2,10 @@
 // gemm_prefill.cu is for bf16.  out[M,N] = sum over 128-wide K blocks of  sa[row,kb] sw[n / 128,kb] (X W^T)_kb,  the scales applied by
 // the block-scaled MMA, one fp32 accumulator over the whole K range.
 //
-// One CTA per SM walks 128 x 192 output tiles.  192 columns are the widest tile whose accumulator fits tensor memory twice (2 x 192
-// of 512 columns) next to the scales in flight (2 x 12), so a tile's epilogue runs under the next tile's MMAs; an instruction of
-// 128 x 192 x 32 asks shared memory for 107 bytes a clock of its 128 (a square tile of 128 for all 128).
+// One CTA per SM walks 128 x 192 output tiles, with the accumulator in tensor memory twice, so that a tile's epilogue runs under the next
+// tile's MMAs.  192 columns are the widest multiple of the 32 that the epilogue loads at once with which five stages fit shared memory
+// (42 KiB each; 224 columns leave room for four).  Wider tiles ask less of shared memory: per MMA it reads 128 + 192 rows for 128 x 192
+// results, a square tile of 128 a fifth more for each.
 //   warp 0 TMA producer (5 stages of 128 K elements), warp 1 MMA issuer, warps 2-5 epilogue
 //   warps 6-9 scales: each stage carries a 512-byte block of row scales and two of column scales (a tile's columns lie in two
 //   128-row blocks of the weight), written next to the operands eight K blocks ahead of the loads' latency
