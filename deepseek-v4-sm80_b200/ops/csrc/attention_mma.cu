@@ -18,8 +18,8 @@
 //
 // What bounds it: the chain gather -> S -> softmax -> PV of a tile, and a token's epilogue, whose stores share the load/store path with
 // the next gather; shared memory feeds an instruction of 64 columns at two thirds of the tensor core's rate.  8 prompts of 1 024
-// tokens (4:1 entries): 800 us, against 2 340 us on the warp-level kernel (attention.cu), which spends four barriers on every 32 keys;
-// 128 decoded tokens at 2 000: 40 and 87 us; one token: 16 and 51 us.
+// tokens (4:1 entries): 840 us, against 2 340 us on the warp-level kernel (attention.cu), which spends four barriers on every 32 keys;
+// 128 decoded tokens at 2 000: 43 and 87 us; one token: 16 and 51 us.
 // The warp-level kernel stays for 8 to 32 heads, where columns would be padding.
 //
 // Splits leave unnormalised sums (fp32) with (reference, sum) per head; a second kernel merges them, four heads to a CTA.
